@@ -163,10 +163,6 @@ int cached_tile_map(CUtensorMap* tm, const void* base, int64_t rows, int64_t wid
 
 }  // namespace
 
-#ifdef DTB_FLASH_TIMING
-namespace dtb { cudaError_t read_flash_timing(long long* host, int n, int head_dim); }
-#endif
-
 extern "C" {
 
 DTB_API int dtb_version(void) { return 100; }
@@ -302,7 +298,7 @@ static int flash_fwd_impl(const void* q, const void* k, const void* v,
   CUtensorMap tq, tk, tv;
   // A tensor map needs at least one row; an empty key chunk never issues a load.
   const int64_t rows_k = total_k > 0 ? total_k : 1;
-  const int kv_rows = dtb::flash_kv_box_rows(head_dim);
+  const int kv_rows = dtb::flash_kv_box_rows();
   if ((rc = cached_tile_map(&tq, q, total_q, width, q_tok_stride, 128, "q")) != DTB_OK) return rc;
   if ((rc = cached_tile_map(&tk, k, rows_k, width, k_tok_stride, kv_rows, "k")) != DTB_OK) return rc;
   if ((rc = cached_tile_map(&tv, v, rows_k, width, v_tok_stride, kv_rows, "v")) != DTB_OK) return rc;
@@ -443,11 +439,5 @@ DTB_API int dtb_drift_accumulate(const float* cur, const float* prev, int64_t n,
   if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_drift_accumulate launch failed: %s", cudaGetErrorString(e));
   return DTB_OK;
 }
-
-#ifdef DTB_FLASH_TIMING
-DTB_API int dtb_debug_flash_timing(long long* host, int n, int head_dim) {
-  return dtb::read_flash_timing(host, n, head_dim) == cudaSuccess ? 0 : DTB_ERR_CUDA;
-}
-#endif
 
 }  // extern "C"

@@ -1,6 +1,5 @@
-// Pieces shared by the two partial-attention forward kernels (flash_fwd_row.cu: one thread per query row,
-// flash_fwd_pair.cu: two threads per query row): tile geometry, the bounded barrier wait, the status word,
-// packed fp32 arithmetic, the lse layouts, and the development-time phase stamps.
+// Pieces of the partial-attention forward kernel (flash_fwd_sm100.cu) that are not its schedule: tile geometry, the
+// bounded barrier wait, the status word, packed fp32 arithmetic, the two exponentials, the lse layouts, the epilogue.
 #pragma once
 #include "flash_fwd_sm100.cuh"
 #include "ptx_sm100.cuh"
@@ -12,9 +11,8 @@ namespace flash {
 
 constexpr int kBM = 128;                  // query rows per tile
 constexpr int kQT = 2;                    // query tiles per CTA
-constexpr int kBN = 64;                   // key rows per tile
-constexpr int kSlabBytes = 128 * 128;     // one TMA box of Q: 128 rows x 64 bf16, 128-byte swizzled
-constexpr int kKvSlabBytes = kBN * 128;   // one TMA box of K / V: 64 rows x 64 bf16
+constexpr int kBN = 128;                  // key rows per tile
+constexpr int kSlabBytes = 128 * 128;     // one TMA box: 128 rows x 64 bf16, 128-byte swizzled
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f; // log2 units: the running reference follows the maximum this lazily
 
@@ -22,13 +20,14 @@ __device__ __forceinline__ void report(int* status, int code) { atomicCAS(status
 
 // Bounded wait that also gives up as soon as any CTA has reported a failure.
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
-    if (((++spins) & 0xff) == 0) {
+    if (((++spins) & 0x3f) == 0) {          // (the clock is read late: most waits end within a few attempts)
       if (*reinterpret_cast<volatile int*>(status) != 0) return false;
-      if (globaltimer_ns() - t0 > 1000000000ull) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > 1000000000ull) {
         report(status, code);
         return false;
       }
@@ -55,6 +54,42 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// 2^x for a pair of exponents, on the ex2 unit ...
+__device__ __forceinline__ uint64_t exp2_mufu2(uint64_t x) {
+  float x0, x1;
+  unpack2(x, x0, x1);
+  return pack2(ex2(x0), ex2(x1));
+}
+
+// ... and on the FMA units, for x <= 127: x = n + f with n = round(x), 2^f on [-1/2, 1/2] by a degree-5 polynomial
+// (least maximum relative error 9.1e-8 with p(0) = 1, weighted least squares iterated to equal ripple), 2^n by
+// placing n + 127 in the exponent field.  Below -127 the result is 0; a NaN stays a NaN.
+__device__ __forceinline__ uint64_t exp2_poly2(uint64_t x) {
+  float x0, x1;
+  unpack2(x, x0, x1);
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x0) : "f"(-127.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x1) : "f"(-127.f));
+  x = pack2(x0, x1);
+  constexpr float kMagic = 12582912.f + 127.f;       // 1.5 * 2^23: the sum's low bits hold n + 127
+  const uint64_t t = add2(x, pack2(kMagic, kMagic));
+  const uint64_t n = add2(t, pack2(-kMagic, -kMagic));
+  const uint64_t f = fma2(n, pack2(-1.f, -1.f), x);
+  uint64_t h = fma2(f, pack2(1.32646751e-3f, 1.32646751e-3f), pack2(9.67151e-3f, 9.67151e-3f));
+  h = fma2(h, f, pack2(5.550734e-2f, 5.550734e-2f));
+  h = fma2(h, f, pack2(2.4022242e-1f, 2.4022242e-1f));
+  h = fma2(h, f, pack2(6.9314698e-1f, 6.9314698e-1f));
+  h = fma2(h, f, pack2(1.f, 1.f));
+  float t0, t1;
+  unpack2(t, t0, t1);
+  const uint64_t scale = pack2(__uint_as_float(__float_as_uint(t0) << 23), __uint_as_float(__float_as_uint(t1) << 23));
+  return mul2(h, scale);
 }
 
 __device__ __forceinline__ int64_t lse_index(const FlashParams& p, int seg, int head, int q_pos, int64_t tok) {
@@ -156,18 +191,5 @@ inline cudaError_t launch_attention_kernel(void (*kernel)(KArgs...), dim3 grid, 
 }
 
 }  // namespace flash
-
-#ifdef DTB_FLASH_TIMING
-// Development aid: per-phase SM clock stamps of one CTA, timing[role][key tile j < 48][phase], read back with
-// dtb_debug_flash_timing (exported only in this build).  Roles 0, 1: first softmax warp of each Q tile;
-// role 2: the MMA issuer.
-#define DTB_STAMP(table, role, j, phase)                                                               \
-  do {                                                                                                 \
-    if (blockIdx.x == 1 && blockIdx.y == 0 && blockIdx.z == 0 && (j) < 48)                             \
-      table[((role) * 48 + (j)) * 8 + (phase)] = clock64();                                            \
-  } while (0)
-#else
-#define DTB_STAMP(table, role, j, phase) do { } while (0)
-#endif
 
 }  // namespace dtb

@@ -1,5 +1,4 @@
-// Parameters and launcher of the partial-attention forward kernels (flash_fwd_sm100.cu picks between
-// flash_fwd_row.cu and flash_fwd_pair.cu by head dimension).
+// Parameters and launcher of the partial-attention forward kernel (flash_fwd_sm100.cu).
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -37,6 +36,6 @@ cudaError_t launch_flash(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const
 
 // Rows of one K / V tile: the tensor maps of k and v must be encoded with boxes of 64 x this many elements
 // (q always uses 64 x 128).
-int flash_kv_box_rows(int head_dim);
+int flash_kv_box_rows();
 
 }  // namespace dtb

@@ -1,0 +1,73 @@
+"""The attention kernel at the sizes where its 128-key tiles, its two-part hand-over and its polynomial exponentials can go
+wrong, against softmax in 64 bits.
+
+Tolerances: probabilities are rounded to bf16 (relative 2^-9) before they meet V, so a result differs from exact by at
+most 2^-9 of the largest |V| of its row plus fp32 accumulation, here 2^-8 in all.  lse is fp32: the exponentials carry a
+relative error below 3e-7 (either unit) and the sum's rounding is of the same order, so |d lse| <= 1e-6 (1 + |lse|)."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _qkv(B, Sq, Sk, H, D, scale=1.0, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    q, k, v = (torch.randn(B, S, H, D, generator=g) for S in (Sq, Sk, Sk))
+    return (q * scale).to(torch.bfloat16).cuda(), k.to(torch.bfloat16).cuda(), v.to(torch.bfloat16).cuda()
+
+
+def _exact(q, k, v):
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) / math.sqrt(q.shape[-1])
+    return torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v.double()), torch.logsumexp(s, -1)
+
+
+def _check(got, want, v):
+    (o, l), (ro, rl) = got, want
+    assert (o.double() - ro).abs().max() <= v.double().abs().max() * 2.0 ** -8
+    assert ((l.double() - rl).abs() <= 1e-6 * (1 + rl.abs())).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,scale", [
+    (1, 1, 1.0), (127, 63, 1.0), (128, 64, 1.0), (129, 65, 1.0), (255, 127, 4.0), (256, 128, 1.0), (257, 129, 1.0),
+    (300, 191, 1.0), (100, 192, 8.0), (513, 255, 1.0), (64, 256, 30.0), (200, 257, 1.0), (256, 384, 100.0), (130, 1409, 1.0)])
+def test_tile_edges(D, Sq, Sk, scale):
+    from ditango_b200 import ops
+    q, k, v = _qkv(2, Sq, Sk, 3, D, scale)
+    want = _exact(q, k, v)
+    _check(ops.flash_partial(q, k, v), want, v)
+    if Sk > 1:                                    # the same keys in two launches, the second merged into the first
+        h = Sk // 3 + 1
+        a, b, c, d = (x.contiguous() for x in (k[:, :h], v[:, :h], k[:, h:], v[:, h:]))
+        o, l = ops.flash_partial(q, a, b)
+        if c.shape[1]:
+            ops.flash_partial(q, c, d, out=o, lse=l, accumulate=True, overlap_previous=True)
+        _check((o, l), want, v)
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_rising_scores_rescale_at_every_tile(D):
+    """Scores that rise by more than 2^8 with every key tile."""
+    from ditango_b200 import ops
+    q, k, v = _qkv(1, 256, 640, 2, D)
+    q = torch.ones_like(q)
+    step = torch.arange(640, device="cuda") // 128
+    for gain in (0.25, 3.0):
+        kk = (k.float() * 0.01 + (gain * 12.0 / math.sqrt(D)) * step[None, :, None, None]).to(torch.bfloat16)
+        _check(ops.flash_partial(q, kk, v), _exact(q, kk, v), v)
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("key", range(112, 144))
+def test_a_nan_key_reaches_every_row(D, key):
+    """Whichever unit exponentiates a column, a NaN score must not turn into a weight of zero."""
+    from ditango_b200 import ops
+    q, k, v = _qkv(1, 130, 200, 1, D)
+    k[0, key, 0, 3] = float("nan")
+    o, l = ops.flash_partial(q, k, v)
+    assert torch.isnan(o).all() and torch.isnan(l).all()
+    assert ops.read_status() == 0
