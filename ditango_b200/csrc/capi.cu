@@ -6,6 +6,7 @@
 #include "drift_stats.cuh"
 #include "errors.cuh"
 #include "merge_states.cuh"
+#include "norm_rope.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -418,6 +419,43 @@ DTB_API int dtb_copy_chunks(int npairs, const void* const* srcs, void* const* ds
   if (n0 * n1 * n2 == 0) return DTB_OK;
   cudaError_t e = dtb::launch_copy_chunks(p, npairs, d->sm_count, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_copy_chunks launch failed: %s", cudaGetErrorString(e));
+  return DTB_OK;
+}
+
+DTB_API int dtb_norm_rope(const void* q, void* q_out, const void* q_weight, const void* q_bias, float q_eps,
+                          const void* k, void* k_out, const void* k_weight, const void* k_bias, float k_eps,
+                          const float* cos, const float* sin,
+                          int batch, int seq, int text_len, int num_heads, int head_dim, void* stream) {
+  if (!q || !q_out || !q_weight || !q_bias || !k || !k_out || !k_weight || !k_bias) return fail(DTB_ERR_ARG, "dtb_norm_rope: null tensor pointer");
+  if (head_dim != 64 && head_dim != 128) return fail(DTB_ERR_ARG, "dtb_norm_rope: head_dim %d not in {64, 128}", head_dim);
+  if (batch < 0 || seq < 0 || num_heads < 1 || text_len < 0 || text_len > seq) return fail(DTB_ERR_ARG, "dtb_norm_rope: bad shape");
+  if (text_len < seq && (!cos || !sin)) return fail(DTB_ERR_ARG, "dtb_norm_rope: null rotary table");
+  const void* all[10] = {q, q_out, q_weight, q_bias, k, k_out, k_weight, k_bias, cos, sin};
+  for (const void* x : all)
+    if (!aligned16(x)) return fail(DTB_ERR_ARG, "dtb_norm_rope: pointers must be 16-byte aligned");
+  DeviceInfo* d = nullptr;
+  int rc = device_info(&d);
+  if (rc != DTB_OK) return rc;
+  dtb::NormRopeParams p;
+  p.src[0] = static_cast<const uint16_t*>(q);
+  p.src[1] = static_cast<const uint16_t*>(k);
+  p.dst[0] = static_cast<uint16_t*>(q_out);
+  p.dst[1] = static_cast<uint16_t*>(k_out);
+  p.weight[0] = static_cast<const uint16_t*>(q_weight);
+  p.weight[1] = static_cast<const uint16_t*>(k_weight);
+  p.bias[0] = static_cast<const uint16_t*>(q_bias);
+  p.bias[1] = static_cast<const uint16_t*>(k_bias);
+  p.cos = cos;
+  p.sin = sin;
+  p.eps[0] = q_eps;
+  p.eps[1] = k_eps;
+  p.tokens = static_cast<int64_t>(batch) * seq;
+  p.seq = seq;
+  p.text_len = text_len;
+  p.num_heads = num_heads;
+  if (p.tokens == 0) return DTB_OK;
+  cudaError_t e = dtb::launch_norm_rope(p, head_dim, d->sm_count, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_norm_rope launch failed: %s", cudaGetErrorString(e));
   return DTB_OK;
 }
 

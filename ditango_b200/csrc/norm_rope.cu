@@ -1,0 +1,119 @@
+// Per-head layer norm of the query and key projections with rotary embedding of the video tokens, one pass.
+//
+// What it replaces in the transformer is a chain of about a dozen elementwise passes per tensor (norm, cast, split,
+// rotate, stack, two products, sum, cast, concatenation), most of them over fp32 copies.  Bound by HBM: each value is
+// read once and written once (bf16).  A token's H heads are handled by one CTA: D/8 lanes own a head (one 16-byte
+// access each), the rotary pairs lie inside a lane, the mean and the variance are shuffles inside the D/8 lanes, and
+// the token's row of the cos / sin tables is read once and kept in registers for all its heads.
+// Measured at 2 x 17776 tokens x 48 heads x 64: 180 us for both tensors (874 MB, 4.9 TB/s); the chain it replaces took
+// about 10 ms, half of it in a layer norm that spends a whole warp's reduction on 64 values.
+#include "norm_rope.cuh"
+
+#include "ptx_sm100.cuh"
+
+namespace dtb {
+
+namespace {
+
+constexpr int kThreads = 128;
+
+__device__ __forceinline__ void unpack8(uint4 v, float (&x)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    x[2 * i] = __uint_as_float(w[i] << 16);
+    x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+}  // namespace
+
+template <int D>
+__global__ void __launch_bounds__(kThreads) norm_rope_kernel(const NormRopeParams p) {
+  constexpr int kLanes = D / 8;           // lanes per head
+  constexpr int kHeadsPerPass = kThreads / kLanes;
+  constexpr int U = 3;                    // passes whose loads are in flight together
+  // (selects, not indexing: a dynamic index would put the parameters into local memory)
+  const bool second = blockIdx.y != 0;
+  const uint16_t* src = second ? p.src[1] : p.src[0];
+  uint16_t* dst = second ? p.dst[1] : p.dst[0];
+  const uint16_t* weight = second ? p.weight[1] : p.weight[0];
+  const uint16_t* bias = second ? p.bias[1] : p.bias[0];
+  const float eps = second ? p.eps[1] : p.eps[0];
+  const int col = (threadIdx.x % kLanes) * 8;
+  const int head0 = threadIdx.x / kLanes;
+  float w[8], b[8];
+  unpack8(*reinterpret_cast<const uint4*>(weight + col), w);
+  unpack8(*reinterpret_cast<const uint4*>(bias + col), b);
+
+  for (int64_t tok = blockIdx.x; tok < p.tokens; tok += gridDim.x) {
+    const int s = static_cast<int>(tok % p.seq);
+    const bool rotate = s >= p.text_len;
+    float cs[8], sn[8];
+    if (rotate) {
+      const int64_t t = static_cast<int64_t>(s - p.text_len) * D + col;
+#pragma unroll
+      for (int i = 0; i < 8; i += 4) {
+        const float4 c4 = *reinterpret_cast<const float4*>(p.cos + t + i);
+        const float4 s4 = *reinterpret_cast<const float4*>(p.sin + t + i);
+        cs[i] = c4.x; cs[i + 1] = c4.y; cs[i + 2] = c4.z; cs[i + 3] = c4.w;
+        sn[i] = s4.x; sn[i + 1] = s4.y; sn[i + 2] = s4.z; sn[i + 3] = s4.w;
+      }
+    }
+    const int64_t base = tok * p.num_heads * D + col;
+    for (int h0 = 0; h0 < p.num_heads; h0 += U * kHeadsPerPass) {
+      uint4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int h = h0 + u * kHeadsPerPass + head0;
+        v[u] = h < p.num_heads ? __ldcs(reinterpret_cast<const uint4*>(src + base + static_cast<int64_t>(h) * D)) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int h = h0 + u * kHeadsPerPass + head0;
+        float x[8];
+        unpack8(v[u], x);
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += x[i];
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, kLanes);
+        const float mean = sum * (1.f / D);
+        float sq = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          x[i] -= mean;
+          sq = fmaf(x[i], x[i], sq);
+        }
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o, kLanes);
+        const float rstd = rsqrtf(sq * (1.f / D) + eps);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = fmaf(x[i] * rstd, w[i], b[i]);
+        if (rotate) {
+#pragma unroll
+          for (int i = 0; i < 8; i += 2) {
+            const float re = x[i], im = x[i + 1];
+            x[i] = re * cs[i] - im * sn[i];
+            x[i + 1] = im * cs[i + 1] + re * sn[i + 1];
+          }
+        }
+        if (h < p.num_heads)
+          *reinterpret_cast<uint4*>(dst + base + static_cast<int64_t>(h) * D) =
+              make_uint4(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]), pack_bf16x2(x[4], x[5]), pack_bf16x2(x[6], x[7]));
+      }
+    }
+  }
+}
+
+cudaError_t launch_norm_rope(const NormRopeParams& p, int head_dim, int sm_count, cudaStream_t stream) {
+  const int64_t cap = static_cast<int64_t>(sm_count) * 8;       // 2 x 8 CTAs of 128 threads per SM, both tensors
+  const dim3 grid(static_cast<unsigned>(p.tokens < cap ? p.tokens : cap), 2);
+  if (head_dim == 64)
+    norm_rope_kernel<64><<<grid, kThreads, 0, stream>>>(p);
+  else
+    norm_rope_kernel<128><<<grid, kThreads, 0, stream>>>(p);
+  return cudaGetLastError();
+}
+
+}  // namespace dtb

@@ -238,6 +238,32 @@ def copy_chunks(pairs: Sequence[Tuple[torch.Tensor, torch.Tensor]], chunk_bytes:
     LaunchLog.count += 1
 
 
+def norm_rope(q: torch.Tensor, k: torch.Tensor, q_norm: Tuple[torch.Tensor, torch.Tensor, float],
+              k_norm: Tuple[torch.Tensor, torch.Tensor, float], cos: torch.Tensor, sin: torch.Tensor,
+              text_len: int) -> Tuple[torch.Tensor, torch.Tensor]:
+    """Layer norm over D of q, k [B,S,H,D] bf16 (norms as (weight, bias, eps)), then rotary embedding (interleaved
+    pairs, cos / sin fp32 [S - text_len, D]) of the tokens behind the first text_len; new tensors, one launch."""
+    lib = _capi.load()
+    _need_cuda(q, k, q_norm[0], q_norm[1], k_norm[0], k_norm[1], cos, sin)
+    B, S, H, D = q.shape
+    for x in (q, k, q_norm[0], q_norm[1], k_norm[0], k_norm[1]):
+        if x.dtype != torch.bfloat16 or not x.is_contiguous():
+            raise _capi.ExtensionError("norm_rope takes contiguous bfloat16 tensors")
+    for x in (cos, sin):
+        if x.dtype != torch.float32 or not x.is_contiguous() or tuple(x.shape) != (S - text_len, D):
+            raise _capi.ExtensionError("cos and sin must be contiguous fp32 tensors of shape [S - text_len, D]")
+    if k.shape != q.shape or any(x.numel() != D for x in (q_norm[0], q_norm[1], k_norm[0], k_norm[1])):
+        raise _capi.ExtensionError("q and k must have one shape; weights and biases hold D elements")
+    qo, ko = torch.empty_like(q), torch.empty_like(k)
+    rc = lib.dtb_norm_rope(
+        q.data_ptr(), qo.data_ptr(), q_norm[0].data_ptr(), q_norm[1].data_ptr(), float(q_norm[2]),
+        k.data_ptr(), ko.data_ptr(), k_norm[0].data_ptr(), k_norm[1].data_ptr(), float(k_norm[2]),
+        cos.data_ptr(), sin.data_ptr(), B, S, text_len, H, D, _stream_ptr())
+    _capi.check(rc, "dtb_norm_rope")
+    LaunchLog.count += 1
+    return qo, ko
+
+
 _DRIFT_SCRATCH = {}
 
 

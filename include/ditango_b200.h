@@ -189,6 +189,21 @@ DTB_API int dtb_copy_chunks(int npairs, const void* const* srcs, void* const* ds
                     int64_t ds0, int64_t ds1, int64_t ds2, void* stream);
 
 /*
+ * Layer norm over each head of the query and key projections, then rotary embedding (interleaved channel
+ * pairs) of the tokens behind the first text_len of every sequence; fp32 arithmetic, one rounding to bf16.
+ * The norm_q / norm_k / apply_rotary_emb steps of the attention adapter
+ * (executor/cogvideox/attention_processor.py:50-72) for both tensors in one launch.
+ *
+ *  q, k           bf16 [batch, seq, num_heads, head_dim] contiguous; q_out, k_out likewise (may be q, k)
+ *  q_weight, ...  bf16 [head_dim]
+ *  cos, sin       fp32 [seq - text_len, head_dim] contiguous; not read when text_len == seq
+ */
+DTB_API int dtb_norm_rope(const void* q, void* q_out, const void* q_weight, const void* q_bias, float q_eps,
+                          const void* k, void* k_out, const void* k_weight, const void* k_bias, float k_eps,
+                          const float* cos, const float* sin,
+                          int batch, int seq, int text_len, int num_heads, int head_dim, void* stream);
+
+/*
  * Drift metric of the redundancy-profiling pass, accumulated on the device:
  *     *accum += mean|cur - prev| / (mean|prev| + 1e-8)      over positions where neither is NaN
  * (mean|cur| instead when mean|prev| < 1e-6; +inf when no position is valid).  Replaces rel_l1

@@ -1,0 +1,54 @@
+"""The fused query / key norm + rotary kernel against the same steps in 64 bits.
+
+Inputs are the same bf16 values; the kernel rounds once, to bf16: half a unit in the last place is 2^-9 relative, and the
+fp32 arithmetic before it adds about 1e-6 of the row's scale."""
+import pytest
+import torch
+import torch.nn as nn
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(x, w, b, eps, cos, sin, text_len):
+    x = x.double()
+    x = (x - x.mean(-1, keepdim=True)) * torch.rsqrt(x.var(-1, unbiased=False, keepdim=True) + eps) * w.double() + b.double()
+    v = x[:, text_len:]
+    rot = torch.stack([-v[..., 1::2], v[..., 0::2]], dim=-1).flatten(-2)
+    v = v * cos.double()[None, :, None] + rot * sin.double()[None, :, None]
+    return torch.cat([x[:, :text_len], v], dim=1)
+
+
+@pytest.mark.parametrize("B,S,H,D,text_len", [(1, 1, 1, 64, 0), (1, 1, 1, 128, 1), (2, 37, 3, 64, 5), (2, 33, 7, 128, 33),
+                                              (1, 300, 48, 64, 226), (2, 129, 50, 64, 0), (1, 65, 24, 128, 17), (1, 2500, 2, 64, 9)])
+def test_norm_rope_matches_exact(B, S, H, D, text_len):
+    from ditango_b200 import ops
+    g = torch.Generator().manual_seed(S)
+    q, k = ((torch.randn(B, S, H, D, generator=g) * 2 + 0.5).to(torch.bfloat16).cuda() for _ in range(2))
+    qn, kn = ((torch.randn(D, generator=g).to(torch.bfloat16).cuda(), torch.randn(D, generator=g).to(torch.bfloat16).cuda(), e)
+              for e in (1e-6, 1e-3))
+    ang = torch.randn(S - text_len, D, generator=g) * 3
+    cos, sin = ang.cos().cuda(), ang.sin().cuda()
+    qo, ko = ops.norm_rope(q, k, qn, kn, cos, sin, text_len)
+    for got, x, n in ((qo, q, qn), (ko, k, kn)):
+        want = _exact(x, n[0], n[1], n[2], cos, sin, text_len)
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+
+
+def test_the_fused_path_and_the_general_one_agree_and_hooks_keep_the_general_one():
+    from ditango_b200 import ops
+    from ditango_b200.executor.cogvideox_dit import norm_and_rotate
+    torch.manual_seed(0)
+    q, k = (torch.randn(2, 50, 4, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    nq, nk = (nn.LayerNorm(64, eps=1e-6).cuda().to(torch.bfloat16) for _ in range(2))
+    ang = torch.randn(44, 64, device="cuda")
+    with torch.no_grad():
+        n0 = ops.LaunchLog.count
+        fused = norm_and_rotate(q, k, nq, nk, ang.cos(), ang.sin(), 6)
+        assert ops.LaunchLog.count == n0 + 1
+        seen = []
+        nk.register_forward_hook(lambda m, i, o: seen.append(1))
+        plain = norm_and_rotate(q, k, nq, nk, ang.cos(), ang.sin(), 6)
+        assert ops.LaunchLog.count == n0 + 1 and seen
+        strided = norm_and_rotate(q.transpose(1, 2).contiguous().transpose(1, 2), k, nq, nk, ang.cos(), ang.sin(), 6)
+    for a, b, c in zip(fused, plain, strided):       # the general path rounds to bf16 twice more
+        assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max() and torch.equal(b, c)
