@@ -1,44 +1,61 @@
 // N-way merge of partial softmax-attention states in one pass over HBM.
 //
 // A "row" is one (token, head) pair: D values per state plus one log-sum-exp per state.  A group of
-// D/4 lanes owns a row (4 fp32 or 4 bf16 values per lane, 128-bit / 64-bit accesses); lane i of the
-// group fetches lse_i, the group reduces max and sum with shuffles, and every lane then pulls the
-// weight of state i from lane i.
+// D/8 lanes owns a row (8 values per lane: two 128-bit accesses in fp32, one in bf16); lane i of the
+// group fetches lse_i (and lse_{i + D/8}), the group reduces max and sum with shuffles, and every lane
+// then pulls the weight of state i from the lane that holds it.
 // Traffic per row: reads sum_i (D * sizeof(state i) + 4) bytes, writes 4*D + 4 (+ 2*D) bytes.
+//
+// A state is kept as loaded (raw bits) until its weight is known.  Its type is only known at run time, so the
+// fp32 and the bf16 load sit in different branches; converting there would make each branch wait for its own load,
+// and the loads of several states would queue behind one another instead of being in flight together (four lanes of 4
+// values with the conversion at the load: fp32 + bf16 at 14882 x 24 x 128 136 us, seven bf16 states and one fp32 at
+// 2 x 6851 x 48 x 128 756 us; as it stands 79 us and about 430 us).
 #include "merge_states.cuh"
 
-#include <cuda_bf16.h>
 #include <math.h>
 
 namespace dtb {
 
 namespace {
 
-__device__ __forceinline__ float4 ld_f4(const float* p) {
-  float4 v;
-  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(p));
+// 8 consecutive values of one state: fp32 in a and b, or bf16 in a.
+struct Raw8 {
+  uint4 a, b;
+};
+
+__device__ __forceinline__ uint4 ld_stream(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
-__device__ __forceinline__ float4 ld_bf4(const uint16_t* p) {
-  uint32_t a, b;
-  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "l"(p));
-  float4 v;
-  v.x = __uint_as_float(a << 16);
-  v.y = __uint_as_float(a & 0xffff0000u);
-  v.z = __uint_as_float(b << 16);
-  v.w = __uint_as_float(b & 0xffff0000u);
-  return v;
+__device__ __forceinline__ void st_stream(void* p, uint4 v) {
+  asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ void st_f4(float* p, float4 v) {
-  asm volatile("st.global.cs.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
 }
-__device__ __forceinline__ void st_bf4(uint16_t* p, float4 v) {
-  uint32_t a, b;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(a) : "f"(v.y), "f"(v.x));
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b) : "f"(v.w), "f"(v.z));
-  asm volatile("st.global.cs.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(a), "r"(b) : "memory");
+__device__ __forceinline__ uint4 as_bits(const float* v) {
+  return make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+}
+// acc += w * state
+__device__ __forceinline__ void add_weighted(float (&acc)[8], float w, const Raw8& r, bool f32) {
+  const uint32_t a[4] = {r.a.x, r.a.y, r.a.z, r.a.w}, b[4] = {r.b.x, r.b.y, r.b.z, r.b.w};
+  if (f32) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc[i] = fmaf(w, __uint_as_float(a[i]), acc[i]);
+      acc[4 + i] = fmaf(w, __uint_as_float(b[i]), acc[4 + i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc[2 * i] = fmaf(w, __uint_as_float(a[i] << 16), acc[2 * i]);
+      acc[2 * i + 1] = fmaf(w, __uint_as_float(a[i] & 0xffff0000u), acc[2 * i + 1]);
+    }
+  }
 }
 
 // Offset of row = (b*S + s)*H + h in an lse tensor.  Rows fit 32 bits (checked by the launcher), so
@@ -54,13 +71,14 @@ __device__ __forceinline__ uint32_t lse_offset(int layout, uint32_t row, uint32_
 
 }  // namespace
 
-// G = lanes per row = D/4.  U rows per group in flight, states fetched CH at a time: every thread
-// keeps CH*U 16-byte loads outstanding and issues them before it touches the weights, so the lse
+// G = lanes per row = D/8.  U rows per group in flight, states fetched CH at a time: every thread
+// has the loads of CH*U row pieces outstanding and issues them before it touches the weights, so the lse
 // round trip and the value round trips overlap instead of queueing behind one another.
 template <int G, int U, int CH>
 __global__ void __launch_bounds__(128) merge_states_kernel(const MergeParams p) {
-  constexpr int D = G * 4;
+  constexpr int D = G * 8;
   constexpr int kGroupsPerWarp = 32 / G;
+  constexpr int kPerLane = kMergeMaxStates / G;        // states whose lse a lane holds: lane, lane + G
   const int lane_in_group = threadIdx.x % G;
   const int64_t warp_id = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
   const int64_t n_warps = static_cast<int64_t>(gridDim.x) * blockDim.x / 32;
@@ -68,21 +86,23 @@ __global__ void __launch_bounds__(128) merge_states_kernel(const MergeParams p) 
   const unsigned full = 0xffffffffu;
   const int n = p.nstates;
 
-  auto load_chunk = [&](int c0, int64_t base, float4 (&v)[CH][U]) {
+  auto load_chunk = [&](int c0, int64_t base, Raw8 (&v)[CH][U]) {
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
       if (c0 + k < n) {
-        const bool f32 = p.out_dtype[c0 + k] == 0;
+        if (p.out_dtype[c0 + k] == 0) {
+          const float* src = static_cast<const float*>(p.outs[c0 + k]) + lane_in_group * 8;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int64_t row = base + u;
-          if (row < p.rows) {
-            const int64_t off = row * D + lane_in_group * 4;
-            v[k][u] = f32 ? ld_f4(static_cast<const float*>(p.outs[c0 + k]) + off)
-                          : ld_bf4(static_cast<const uint16_t*>(p.outs[c0 + k]) + off);
-          } else {
-            v[k][u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          }
+          for (int u = 0; u < U; ++u)
+            if (base + u < p.rows) {
+              v[k][u].a = ld_stream(src + (base + u) * D);
+              v[k][u].b = ld_stream(src + (base + u) * D + 4);
+            }
+        } else {
+          const uint16_t* src = static_cast<const uint16_t*>(p.outs[c0 + k]) + lane_in_group * 8;
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (base + u < p.rows) v[k][u].a = ld_stream(src + (base + u) * D);
         }
       }
     }
@@ -92,48 +112,61 @@ __global__ void __launch_bounds__(128) merge_states_kernel(const MergeParams p) 
   // past the end are guarded individually.
   for (int64_t wbase = warp_id * kGroupsPerWarp * U; wbase < p.rows; wbase += n_warps * kGroupsPerWarp * U) {
     const int64_t base = wbase + group_in_warp * U;
-    float my[U];
+    float my[U][kPerLane];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int64_t row = base + u;
-      my[u] = -INFINITY;
-      if (row < p.rows && lane_in_group < n)
-        my[u] = p.lse[lane_in_group][lse_offset(p.lse_layout[lane_in_group], static_cast<uint32_t>(row), p.H, p.S)];
-    }
-    float4 v[CH][U];
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int t = 0; t < kPerLane; ++t) {
+        const int st = lane_in_group + t * G;
+        my[u][t] = -INFINITY;
+        if (base + u < p.rows && st < n)
+          my[u][t] = p.lse[st][lse_offset(p.lse_layout[st], static_cast<uint32_t>(base + u), p.H, p.S)];
+      }
+    Raw8 v[CH][U];
+#pragma unroll
+    for (int k = 0; k < CH; ++k)
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[k][u].a = v[k][u].b = make_uint4(0u, 0u, 0u, 0u);
     load_chunk(0, base, v);
 
-    float w[U];        // this lane's weight (state index = lane_in_group)
+    float w[U][kPerLane];        // weights of the states this lane holds the lse of
     float lse_out[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      float mx = my[u];
+      float mx = my[u][0];
+#pragma unroll
+      for (int t = 1; t < kPerLane; ++t) mx = fmaxf(mx, my[u][t]);
 #pragma unroll
       for (int o = G / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(full, mx, o, G));
-      const float e = (my[u] == -INFINITY) ? 0.f : __expf(my[u] - mx);
-      float sum = e;
+      float e[kPerLane], sum = 0.f;
+#pragma unroll
+      for (int t = 0; t < kPerLane; ++t) {
+        e[t] = (my[u][t] == -INFINITY) ? 0.f : __expf(my[u][t] - mx);
+        sum += e[t];
+      }
 #pragma unroll
       for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o, G);
-      w[u] = (sum > 0.f) ? e / sum : 0.f;
+#pragma unroll
+      for (int t = 0; t < kPerLane; ++t) w[u][t] = (sum > 0.f) ? e[t] / sum : 0.f;
       lse_out[u] = (sum > 0.f) ? mx + __logf(sum) : -INFINITY;
     }
-    float4 acc[U];
+    float acc[U][8];
 #pragma unroll
-    for (int u = 0; u < U; ++u) acc[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[u][i] = 0.f;
     for (int c0 = 0; c0 < n; c0 += CH) {
 #pragma unroll
       for (int k = 0; k < CH; ++k) {
-        if (c0 + k < n) {
+        const int st = c0 + k;
+        if (st < n) {
+          const bool f32 = p.out_dtype[st] == 0;
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            const float wi = __shfl_sync(full, w[u], c0 + k, G);
+            const float mine = (kPerLane == 1 || st < G) ? w[u][0] : w[u][kPerLane - 1];
+            const float wi = __shfl_sync(full, mine, st % G, G);
             // a state with weight 0 may hold anything (even inf/nan): it must not reach the sum
-            if (wi != 0.f) {
-              acc[u].x = fmaf(wi, v[k][u].x, acc[u].x);
-              acc[u].y = fmaf(wi, v[k][u].y, acc[u].y);
-              acc[u].z = fmaf(wi, v[k][u].z, acc[u].z);
-              acc[u].w = fmaf(wi, v[k][u].w, acc[u].w);
-            }
+            if (wi != 0.f) add_weighted(acc[u], wi, v[k][u], f32);
           }
         }
       }
@@ -143,9 +176,14 @@ __global__ void __launch_bounds__(128) merge_states_kernel(const MergeParams p) 
     for (int u = 0; u < U; ++u) {
       const int64_t row = base + u;
       if (row < p.rows) {
-        const int64_t off = row * D + lane_in_group * 4;
-        if (p.out != nullptr) st_f4(p.out + off, acc[u]);
-        if (p.out_bf16 != nullptr) st_bf4(p.out_bf16 + off, acc[u]);
+        const int64_t off = row * D + lane_in_group * 8;
+        if (p.out != nullptr) {
+          st_stream(p.out + off, as_bits(acc[u]));
+          st_stream(p.out + off + 4, as_bits(acc[u] + 4));
+        }
+        if (p.out_bf16 != nullptr)
+          st_stream(p.out_bf16 + off, make_uint4(pack_bf16(acc[u][0], acc[u][1]), pack_bf16(acc[u][2], acc[u][3]),
+                                                 pack_bf16(acc[u][4], acc[u][5]), pack_bf16(acc[u][6], acc[u][7])));
         if (p.lse_out != nullptr && lane_in_group == 0)
           p.lse_out[lse_offset(p.lse_out_layout, static_cast<uint32_t>(row), p.H, p.S)] = lse_out[u];
       }
@@ -160,24 +198,24 @@ static cudaError_t launch_merge_cfg(const MergeParams& p, int G, int sm_count, c
   const int64_t blocks_needed = (groups_needed * G + kThreads - 1) / kThreads + 1;
   // one resident wave: CTAs per SM as the occupancy calculator reports them for this instantiation
   int per_sm = 0;
-  cudaError_t oe = (G == 16)
-      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, merge_states_kernel<16, U, CH>, kThreads, 0)
-      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, merge_states_kernel<32, U, CH>, kThreads, 0);
+  cudaError_t oe = (G == 8)
+      ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, merge_states_kernel<8, U, CH>, kThreads, 0)
+      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, merge_states_kernel<16, U, CH>, kThreads, 0);
   if (oe != cudaSuccess || per_sm < 1) per_sm = 6;
   const int64_t cap = static_cast<int64_t>(sm_count) * per_sm;
   int blocks = static_cast<int>(blocks_needed < cap ? blocks_needed : cap);
   if (blocks < 1) blocks = 1;
-  if (G == 16)
-    merge_states_kernel<16, U, CH><<<blocks, kThreads, 0, stream>>>(p);
+  if (G == 8)
+    merge_states_kernel<8, U, CH><<<blocks, kThreads, 0, stream>>>(p);
   else
-    merge_states_kernel<32, U, CH><<<blocks, kThreads, 0, stream>>>(p);
+    merge_states_kernel<16, U, CH><<<blocks, kThreads, 0, stream>>>(p);
   return cudaGetLastError();
 }
 
 // Rows per thread x states per fetch are chosen so that about eight 16-byte loads are outstanding
 // per thread whatever the number of states: 4 rows x 2 states, 3 x 3, or 2 x 4.
 cudaError_t launch_merge(const MergeParams& p, int head_dim, int sm_count, cudaStream_t stream) {
-  const int G = head_dim / 4;
+  const int G = head_dim / 8;
   if (p.rows >= (1ll << 31)) return cudaErrorInvalidValue;
 #ifndef DTB_MERGE_FIXED_CFG
   if (p.nstates <= 2) return launch_merge_cfg<4, 2>(p, G, sm_count, stream);
