@@ -68,7 +68,29 @@ __global__ void __launch_bounds__(kThreads) drift_stats_kernel(const float* __re
   const int64_t tile1 = (tile0 + kDriftTile < n) ? tile0 + kDriftTile : n;
   float d = 0.f, o = 0.f, m = 0.f, k = 0.f;   // <= 64 elements per thread: fp32 is exact enough here
   const bool aligned = ((reinterpret_cast<uintptr_t>(cur) | reinterpret_cast<uintptr_t>(prev)) & 15) == 0;
-  if (aligned) {
+  if (aligned && tile1 - tile0 == kDriftTile) {
+    // Full tiles (all but the last one): the loads of kBatch steps are issued before the first value is used (bound by
+    // HBM; 2 x 27.3 M values 39 us, 5.6 TB/s, against 43 us with one step's loads at a time).
+    const float4* c4 = reinterpret_cast<const float4*>(cur + tile0) + threadIdx.x;
+    const float4* p4 = reinterpret_cast<const float4*>(prev + tile0) + threadIdx.x;
+    constexpr int kBatch = 4;
+#pragma unroll 1
+    for (int s = 0; s < kDriftTile / (kThreads * 4); s += kBatch) {
+      float4 c[kBatch], p[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        c[b] = __ldcs(c4 + (s + b) * kThreads);
+        p[b] = __ldcs(p4 + (s + b) * kThreads);
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        add_elem(c[b].x, p[b].x, d, o, m, k);
+        add_elem(c[b].y, p[b].y, d, o, m, k);
+        add_elem(c[b].z, p[b].z, d, o, m, k);
+        add_elem(c[b].w, p[b].w, d, o, m, k);
+      }
+    }
+  } else if (aligned) {
     for (int64_t i = tile0 + threadIdx.x * 4; i < tile1; i += kThreads * 4) {
       if (i + 4 <= tile1) {
         const float4 c = __ldcs(reinterpret_cast<const float4*>(cur + i));
