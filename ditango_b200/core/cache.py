@@ -28,6 +28,11 @@ def _device_total_mb() -> float:
     return float("inf")
 
 
+def _allocated_bytes() -> int:
+    # torch.cuda.memory_allocated() flattens and sorts every counter of the allocator to return this one
+    return torch.cuda.memory_stats_as_nested_dict().get("allocated_bytes", {}).get("all", {}).get("current", 0)
+
+
 class proCache:
     def __init__(self, isp_size: int, layer_id: int, store_dtype: torch.dtype = torch.float32,
                  lse_layout: int = LSE_BHS):
@@ -119,7 +124,7 @@ class proCache:
         if predicted <= active:
             return True
         add_mb = self.block_size_mb * (predicted - active)
-        cur_mb = torch.cuda.memory_allocated() / (1024 * 1024) if torch.cuda.is_available() else 0.0
+        cur_mb = _allocated_bytes() / (1024 * 1024) if torch.cuda.is_available() else 0.0
         if cur_mb + add_mb > self.memory_constraint:
             logger.warning(f"T{get_timestep()}L{layer_id} | Memory check failed: {cur_mb + add_mb:.0f} MB > "
                            f"{self.memory_constraint:.0f} MB, setting stride {next_isp_stride} to {self.isp_size}")

@@ -32,7 +32,8 @@ class LaunchLog:
 
 
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: building a Stream object around it costs several times the rest of a launch's Python
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _need_cuda(*ts):
@@ -58,7 +59,7 @@ def read_status() -> int:
     return _capi.load().dtb_read_status(_stream_ptr())
 
 
-_STATUS_WATCH = {}      # device index -> [pinned int32 word, event behind the copy in flight or None]
+_STATUS_WATCH = {}      # device index -> [pinned int32 word, event behind the copy in flight or None, the event kept for it]
 
 
 def poll_status():
@@ -71,8 +72,8 @@ def poll_status():
     dev = torch.cuda.current_device()
     watch = _STATUS_WATCH.get(dev)
     if watch is None:
-        watch = _STATUS_WATCH[dev] = [torch.zeros(1, dtype=torch.int32).pin_memory(), None]
-    host, pending = watch
+        watch = _STATUS_WATCH[dev] = [torch.zeros(1, dtype=torch.int32).pin_memory(), None, None]
+    host, pending, _ = watch
     if pending is not None:
         if not pending.query():
             return                       # the earlier copy is still behind queued work
@@ -83,9 +84,10 @@ def poll_status():
                 f"a kernel gave up on a bounded wait (device status {code}); launches since then skipped "
                 "their work -- results are not valid; read_status() clears the word")
     _capi.check(lib.dtb_peek_status_async(host.data_ptr(), _stream_ptr()), "dtb_peek_status_async")
-    ev = torch.cuda.Event()
-    ev.record()
-    watch[1] = ev
+    if watch[2] is None:
+        watch[2] = torch.cuda.Event()
+    watch[2].record()
+    watch[1] = watch[2]
 
 
 def post_status(code: int):
