@@ -22,7 +22,7 @@ EXPORTS = (
     "dtb_peek_status_async", "dtb_post_status",
     "dtb_ipc_export_mem", "dtb_ipc_open_mem", "dtb_ipc_close_mem", "dtb_peer_copy_async",
     "dtb_flash_fwd", "dtb_flash_fwd_ex", "dtb_merge_states", "dtb_copy_chunks",
-    "dtb_norm_rope", "dtb_drift_scratch_bytes", "dtb_drift_accumulate",
+    "dtb_norm_rope", "dtb_ln_modulate", "dtb_gate_add", "dtb_drift_scratch_bytes", "dtb_drift_accumulate",
     "dtb_drift_noalloc_max_elements", "dtb_drift_accumulate_noalloc",
 )
 
@@ -82,6 +82,12 @@ def load():
     lib.dtb_norm_rope.argtypes = [
         c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_float,
         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p]
+    lib.dtb_ln_modulate.restype = c_int
+    lib.dtb_ln_modulate.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p,
+                                    c_int, c_int, c_int, c_int, c_void_p]
+    lib.dtb_gate_add.restype = c_int
+    lib.dtb_gate_add.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                 c_int, c_int, c_int, c_int, c_void_p]
     lib.dtb_drift_scratch_bytes.restype = c_int64
     lib.dtb_drift_scratch_bytes.argtypes = [c_int64]
     lib.dtb_drift_accumulate.restype = c_int

@@ -6,6 +6,7 @@
 #include "drift_stats.cuh"
 #include "errors.cuh"
 #include "merge_states.cuh"
+#include "norm_mod.cuh"
 #include "norm_rope.cuh"
 
 #include <cuda.h>
@@ -15,6 +16,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 
 namespace {
@@ -456,6 +458,63 @@ DTB_API int dtb_norm_rope(const void* q, void* q_out, const void* q_weight, cons
   if (p.tokens == 0) return DTB_OK;
   cudaError_t e = dtb::launch_norm_rope(p, head_dim, d->sm_count, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_norm_rope launch failed: %s", cudaGetErrorString(e));
+  return DTB_OK;
+}
+
+static int check_streams(const char* what, std::initializer_list<const void*> ptrs, int batch, int video_len, int text_len, int dim) {
+  for (const void* x : ptrs) {
+    if (!x) return fail(DTB_ERR_ARG, "%s: null tensor pointer", what);
+    if (!aligned16(x)) return fail(DTB_ERR_ARG, "%s: pointers must be 16-byte aligned", what);
+  }
+  if (batch < 0 || batch > 65535 || video_len < 0 || text_len < 0) return fail(DTB_ERR_ARG, "%s: bad shape", what);
+  if (dim < 256 || dim > dtb::kModMaxDim || dim % 256) return fail(DTB_ERR_ARG, "%s: dim %d is not a multiple of 256 up to %d", what, dim, dtb::kModMaxDim);
+  return DTB_OK;
+}
+
+DTB_API int dtb_ln_modulate(const void* video, const void* text, const void* weight, const void* bias, float eps,
+                            const void* mod, void* out, int batch, int video_len, int text_len, int dim, void* stream) {
+  int rc = check_streams("dtb_ln_modulate", {video, text, weight, bias, mod, out}, batch, video_len, text_len, dim);
+  if (rc != DTB_OK) return rc;
+  DeviceInfo* d = nullptr;
+  if ((rc = device_info(&d)) != DTB_OK) return rc;
+  if (batch == 0 || (video_len == 0 && text_len == 0)) return DTB_OK;
+  dtb::LnModulateParams p;
+  p.video = static_cast<const uint16_t*>(video);
+  p.text = static_cast<const uint16_t*>(text);
+  p.weight = static_cast<const uint16_t*>(weight);
+  p.bias = static_cast<const uint16_t*>(bias);
+  p.mod = static_cast<const uint16_t*>(mod);
+  p.out = static_cast<uint16_t*>(out);
+  p.mod_stride = 6ll * dim;
+  p.eps = eps;
+  p.video_len = video_len;
+  p.text_len = text_len;
+  p.dim = dim;
+  cudaError_t e = dtb::launch_ln_modulate(p, batch, d->sm_count, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_ln_modulate launch failed: %s", cudaGetErrorString(e));
+  return DTB_OK;
+}
+
+DTB_API int dtb_gate_add(const void* video, const void* text, const void* a, const void* mod, void* video_out, void* text_out,
+                         int batch, int video_len, int text_len, int dim, void* stream) {
+  int rc = check_streams("dtb_gate_add", {video, text, a, mod, video_out, text_out}, batch, video_len, text_len, dim);
+  if (rc != DTB_OK) return rc;
+  DeviceInfo* d = nullptr;
+  if ((rc = device_info(&d)) != DTB_OK) return rc;
+  if (batch == 0 || (video_len == 0 && text_len == 0)) return DTB_OK;
+  dtb::GateAddParams p;
+  p.video = static_cast<const uint16_t*>(video);
+  p.text = static_cast<const uint16_t*>(text);
+  p.a = static_cast<const uint16_t*>(a);
+  p.mod = static_cast<const uint16_t*>(mod);
+  p.video_out = static_cast<uint16_t*>(video_out);
+  p.text_out = static_cast<uint16_t*>(text_out);
+  p.mod_stride = 6ll * dim;
+  p.video_len = video_len;
+  p.text_len = text_len;
+  p.dim = dim;
+  cudaError_t e = dtb::launch_gate_add(p, batch, d->sm_count, static_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_gate_add launch failed: %s", cudaGetErrorString(e));
   return DTB_OK;
 }
 

@@ -71,26 +71,35 @@ def apply_rotary(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch
     return (x.float() * cos[None, :, None, :] + rot * sin[None, :, None, :]).to(x.dtype)
 
 
-def _plain_head_norm(norm: nn.Module, head_dim: int, device: torch.device) -> bool:
-    """True for a bf16 LayerNorm over the head's channels that nothing observes: no hook of its own, and its call
-    (which the fused kernel stands in for) not replaced."""
-    return (type(norm) is nn.LayerNorm and tuple(norm.normalized_shape) == (head_dim,) and
+def _unobserved(m: nn.Module, kind: type) -> bool:
+    """True when calling `m` is running kind.forward and nothing else: no subclass, no hook, no replaced forward."""
+    mod = nn.modules.module
+    return (type(m) is kind and "forward" not in m.__dict__ and
+            not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and
+            not (mod._global_forward_hooks or mod._global_forward_pre_hooks or mod._global_backward_hooks or
+                 mod._global_backward_pre_hooks))
+
+
+def _plain_norm(norm: nn.Module, dim: int, device: torch.device) -> bool:
+    """True for a bf16 LayerNorm over the last `dim` channels on `device` that a kernel may stand in for."""
+    return (_unobserved(norm, nn.LayerNorm) and tuple(norm.normalized_shape) == (dim,) and
             norm.weight is not None and norm.bias is not None and norm.weight.dtype == norm.bias.dtype == torch.bfloat16 and
             norm.weight.device == norm.bias.device == device and
-            "forward" not in norm.__dict__ and not norm._forward_hooks and not norm._forward_pre_hooks and
-            not norm._backward_hooks and not norm._backward_pre_hooks)
+            norm.weight.data_ptr() % 16 == 0 and norm.bias.data_ptr() % 16 == 0)
+
+
+def _plain_bf16(device: torch.device, *tensors: torch.Tensor) -> bool:
+    return all(x.dtype == torch.bfloat16 and x.device == device and x.is_contiguous() and x.data_ptr() % 16 == 0 for x in tensors)
 
 
 def norm_and_rotate(q, k, norm_q, norm_k, cos, sin, text_len: int) -> Tuple[torch.Tensor, torch.Tensor]:
     """norm_q / norm_k over the heads of q, k [B, S, H, D], then rotary embedding of the tokens behind the first
     text_len.  On a GPU in bf16 this is one kernel over both tensors (fp32 inside, one rounding at the end)."""
     D = q.shape[-1]
-    if (q.is_cuda and q.dtype == k.dtype == torch.bfloat16 and D in (64, 128) and q.is_contiguous() and k.is_contiguous() and
-            cos.is_contiguous() and sin.is_contiguous() and
-            cos.dtype == sin.dtype == torch.float32 and cos.shape == sin.shape == (q.shape[1] - text_len, D) and
-            _plain_head_norm(norm_q, D, q.device) and _plain_head_norm(norm_k, D, q.device) and
-            all(x.device == q.device and x.data_ptr() % 16 == 0 for x in (q, k, cos, sin, norm_q.weight, norm_q.bias,
-                                                                          norm_k.weight, norm_k.bias)) and
+    if (q.is_cuda and D in (64, 128) and q.shape == k.shape and _plain_bf16(q.device, q, k) and
+            _plain_norm(norm_q, D, q.device) and _plain_norm(norm_k, D, q.device) and
+            all(x.dtype == torch.float32 and x.shape == (q.shape[1] - text_len, D) and x.is_contiguous() and
+                x.device == q.device and x.data_ptr() % 16 == 0 for x in (cos, sin)) and
             not torch.is_autocast_enabled("cuda")):
         return _engine.norm_rope(q, k, (norm_q.weight, norm_q.bias, norm_q.eps), (norm_k.weight, norm_k.bias, norm_k.eps),
                                  cos, sin, text_len)
@@ -105,6 +114,21 @@ class LayerNormZero(nn.Module):
         super().__init__()
         self.linear = nn.Linear(time_dim, 6 * dim)
         self.norm = nn.LayerNorm(dim, eps=1e-5)
+
+    def fuses(self, h, enc) -> bool:
+        """Whether `joint` may stand in for forward(): bf16 streams on a GPU, no gradient to be recorded (the kernels have
+        none), and no hook on the modules whose calls it skips."""
+        dim = h.shape[-1]
+        return (h.is_cuda and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda") and
+                dim % 256 == 0 and dim <= _engine.MOD_MAX_DIM and h.numel() > 0 and enc.numel() > 0 and
+                _plain_bf16(h.device, h, enc) and
+                self.linear.weight.dtype == torch.bfloat16 and
+                _unobserved(self, LayerNormZero) and _plain_norm(self.norm, dim, h.device))
+
+    def joint(self, h, enc, temb):
+        """([B, text + video, dim] normalised and modulated, text first; the modulation, whose gates ops.gate_add takes)."""
+        mod = self.linear(F.silu(temb)).contiguous()
+        return _engine.ln_modulate(h, enc, self.norm.weight, self.norm.bias, self.norm.eps, mod), mod
 
     def forward(self, h, enc, temb):
         shift, scale, gate, e_shift, e_scale, e_gate = self.linear(F.silu(temb)).chunk(6, dim=1)
@@ -147,23 +171,37 @@ class DiTBlock(nn.Module):
             o_enc = sequence_to_heads(out[:, :text_all].contiguous(), self.group).flatten(2).to(h.dtype)
             o_vid = sequence_to_heads(out[:, text_all:].contiguous(), self.group).flatten(2).to(h.dtype)
             return self.to_out(o_vid), self.to_out(o_enc)
-        x = torch.cat([enc, h], dim=1)
+        out = self._attend_joint(torch.cat([enc, h], dim=1), text_len, rope)
+        return out[:, text_len:], out[:, :text_len]
+
+    def _attend_joint(self, x, text_len, rope):
+        """Attention of the joint sequence x [B, text + video, dim], projected back."""
+        B, H, D = x.shape[0], self.cfg.num_heads, self.cfg.head_dim
         q, k, v = (f(x).view(B, -1, H, D) for f in (self.to_q, self.to_k, self.to_v))
         cos, sin = rope                                              # this rank's slice of the tables
         q, k = norm_and_rotate(q, k, self.norm_q, self.norm_k, cos, sin, text_len)
         out = self.attention.attn(q, k, v.contiguous())
-        out = self.to_out(out.to(x.dtype).flatten(2))
-        return out[:, text_len:], out[:, :text_len]
+        return self.to_out(out.to(x.dtype).flatten(2))
 
     def forward(self, h, enc, temb, rope):
         text_len = enc.shape[1]
-        nh, nenc, gate, e_gate = self.norm1(h, enc, temb)
-        a_h, a_enc = self._attend(nh, nenc, rope)
-        h = h + gate * a_h
-        enc = enc + e_gate * a_enc
+        if self.mode != "ulysses" and self.norm1.fuses(h, enc):
+            x, mod = self.norm1.joint(h, enc, temb)
+            h, enc = _engine.gate_add(h, enc, self._attend_joint(x, text_len, rope), mod)
+        else:
+            nh, nenc, gate, e_gate = self.norm1(h, enc, temb)
+            a_h, a_enc = self._attend(nh, nenc, rope)
+            h = h + gate * a_h
+            enc = enc + e_gate * a_enc
+        if self.norm2.fuses(h, enc):
+            x, mod = self.norm2.joint(h, enc, temb)
+            return _engine.gate_add(h, enc, self._feed_forward(x), mod)
         nh, nenc, gate, e_gate = self.norm2(h, enc, temb)
-        ff = self.ff_out(F.gelu(self.ff_in(torch.cat([nenc, nh], dim=1)), approximate="tanh"))
+        ff = self._feed_forward(torch.cat([nenc, nh], dim=1))
         return h + gate * ff[:, text_len:], enc + e_gate * ff[:, :text_len]
+
+    def _feed_forward(self, x):
+        return self.ff_out(F.gelu(self.ff_in(x), approximate="tanh"))
 
 
 class CogVideoXDiT(nn.Module):

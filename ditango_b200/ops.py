@@ -266,6 +266,49 @@ def norm_rope(q: torch.Tensor, k: torch.Tensor, q_norm: Tuple[torch.Tensor, torc
     return qo, ko
 
 
+MOD_MAX_DIM = 3072
+
+
+def _check_streams(video, text, *others):
+    _need_cuda(video, text, *others)
+    B, Sv, dim = video.shape
+    if text.dim() != 3 or text.shape[0] != B or text.shape[2] != dim:
+        raise _capi.ExtensionError("video and text must be [B, S, dim] tensors of one batch and width")
+    for x in (video, text, *others):
+        if x.dtype != torch.bfloat16 or not x.is_contiguous():
+            raise _capi.ExtensionError("contiguous bfloat16 tensors expected")
+    return B, Sv, text.shape[1], dim
+
+
+def ln_modulate(video: torch.Tensor, text: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float,
+                mod: torch.Tensor) -> torch.Tensor:
+    """Layer norm of both streams, modulated by `mod` [B, 6 dim] (shift, scale, gate of video, then of text): the joint
+    tensor [B, text + video, dim], text first, in one launch."""
+    B, Sv, St, dim = _check_streams(video, text, weight, bias, mod)
+    if weight.numel() != dim or bias.numel() != dim or tuple(mod.shape) != (B, 6 * dim):
+        raise _capi.ExtensionError("weight and bias hold dim elements, mod is [B, 6 dim]")
+    out = torch.empty(B, St + Sv, dim, dtype=torch.bfloat16, device=video.device)
+    rc = _capi.load().dtb_ln_modulate(video.data_ptr(), text.data_ptr(), weight.data_ptr(), bias.data_ptr(), float(eps),
+                                      mod.data_ptr(), out.data_ptr(), B, Sv, St, dim, _stream_ptr())
+    _capi.check(rc, "dtb_ln_modulate")
+    LaunchLog.count += 1
+    return out
+
+
+def gate_add(video: torch.Tensor, text: torch.Tensor, a: torch.Tensor, mod: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(video, text) + gate * (their parts of the joint tensor a [B, text + video, dim]), gates from `mod` as in
+    ln_modulate; new tensors, one launch."""
+    B, Sv, St, dim = _check_streams(video, text, a, mod)
+    if tuple(a.shape) != (B, St + Sv, dim) or tuple(mod.shape) != (B, 6 * dim):
+        raise _capi.ExtensionError("a is [B, text + video, dim], mod is [B, 6 dim]")
+    vo, to = torch.empty_like(video), torch.empty_like(text)
+    rc = _capi.load().dtb_gate_add(video.data_ptr(), text.data_ptr(), a.data_ptr(), mod.data_ptr(), vo.data_ptr(), to.data_ptr(),
+                                   B, Sv, St, dim, _stream_ptr())
+    _capi.check(rc, "dtb_gate_add")
+    LaunchLog.count += 1
+    return vo, to
+
+
 _DRIFT_SCRATCH = {}
 
 

@@ -204,6 +204,23 @@ DTB_API int dtb_norm_rope(const void* q, void* q_out, const void* q_weight, cons
                           int batch, int seq, int text_len, int num_heads, int head_dim, void* stream);
 
 /*
+ * The two elementwise steps around a transformer block's sub-layers (LayerNormZero modulation and gated residual,
+ * executor/cogvideox/cogvideox_transformer_3d.py:139-190), over both streams in one launch each; fp32 arithmetic,
+ * one rounding to bf16.  All tensors bf16, contiguous.
+ *
+ *  dtb_ln_modulate   out[b, s] = (LayerNorm(x[b, s]) * weight + bias) * (1 + scale[b]) + shift[b]
+ *  dtb_gate_add      x_out[b, s] = x[b, s] + gate[b] * a[b, s]          (x_out may be x)
+ *
+ *  video, text   [batch, video_len, dim], [batch, text_len, dim]; out, a: [batch, text_len + video_len, dim], text first
+ *  mod           [batch, 6 dim]: shift, scale, gate of the video stream, then of the text stream
+ *  dim           a multiple of 256, at most 3072
+ */
+DTB_API int dtb_ln_modulate(const void* video, const void* text, const void* weight, const void* bias, float eps,
+                            const void* mod, void* out, int batch, int video_len, int text_len, int dim, void* stream);
+DTB_API int dtb_gate_add(const void* video, const void* text, const void* a, const void* mod, void* video_out, void* text_out,
+                         int batch, int video_len, int text_len, int dim, void* stream);
+
+/*
  * Drift metric of the redundancy-profiling pass, accumulated on the device:
  *     *accum += mean|cur - prev| / (mean|prev| + 1e-8)      over positions where neither is NaN
  * (mean|cur| instead when mean|prev| < 1e-6; +inf when no position is valid).  Replaces rel_l1

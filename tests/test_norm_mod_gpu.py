@@ -1,0 +1,69 @@
+"""The fused layer norm + modulation and the gated residual of the transformer block against the same steps in 64 bits.
+
+The kernels round once, to bf16 (2^-9 relative); their fp32 arithmetic adds about 1e-6 of the terms' size."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf16(g, *shape, scale=1.0, shift=0.0):
+    return (torch.randn(*shape, generator=g) * scale + shift).to(torch.bfloat16).cuda()
+
+
+@pytest.mark.parametrize("B,Sv,St,dim", [(1, 1, 1, 256), (2, 9, 3, 512), (1, 8, 16, 768), (2, 333, 226, 3072), (1, 1500, 1, 1536), (3, 40, 77, 2816)])
+def test_ln_modulate_and_gate_add_match_exact(B, Sv, St, dim):
+    from ditango_b200 import ops
+    g = torch.Generator().manual_seed(dim + Sv)
+    video, text = _bf16(g, B, Sv, dim, scale=3.0, shift=0.7), _bf16(g, B, St, dim)
+    w, b, mod = _bf16(g, dim), _bf16(g, dim), _bf16(g, B, 6 * dim)
+    a = _bf16(g, B, St + Sv, dim)
+    m = mod.double().view(B, 6, 1, dim)
+
+    def norm(x, shift, scale):
+        x = x.double()
+        x = (x - x.mean(-1, keepdim=True)) * torch.rsqrt(x.var(-1, unbiased=False, keepdim=True) + 1e-5) * w.double() + b.double()
+        return x * (1 + scale) + shift
+
+    got = ops.ln_modulate(video, text, w, b, 1e-5, mod).double()
+    want = torch.cat([norm(text, m[:, 3], m[:, 4]), norm(video, m[:, 0], m[:, 1])], dim=1)
+    assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all()
+    gv, gt = ops.gate_add(video, text, a, mod)
+    assert ((gv.double() - (video.double() + m[:, 2] * a[:, St:].double())).abs() <= gv.double().abs() * 2.0 ** -8 + 1e-5).all()
+    assert ((gt.double() - (text.double() + m[:, 5] * a[:, :St].double())).abs() <= gt.double().abs() * 2.0 ** -8 + 1e-5).all()
+
+
+def test_block_takes_the_fused_path_only_where_nothing_observes_it():
+    from ditango_b200 import ops
+    from ditango_b200.core import redundancy_map as rmod
+    from ditango_b200.core.config import init_config
+    from ditango_b200.core.group_coordinate import SingleRankGroup
+    from ditango_b200.executor.cogvideox_dit import DiTBlock, DiTConfig
+    from ditango_b200.utils import update_timestep
+    cfg = init_config(None, make_output_dir=False)
+    cfg.num_layers, cfg.num_inference_steps = 1, 1
+    rmod.destroy_redundancy_map()
+    rmod.init_redundancy_map(cfg, world_size=1)
+    update_timestep(0)
+    torch.manual_seed(0)
+    dc = DiTConfig(num_layers=1, num_heads=4, frames=1, height=8, width=8, text_len=5)
+    block = DiTBlock(dc, 0, SingleRankGroup(torch.device("cuda", 0)), "ditango").cuda().to(torch.bfloat16)
+    h, enc, temb = (torch.randn(s, device="cuda").to(torch.bfloat16) for s in ((2, 16, 256), (2, 5, 256), (2, 512)))
+    rope = (torch.ones(16, 64, device="cuda"), torch.zeros(16, 64, device="cuda"))
+    with torch.no_grad():
+        n0 = ops.LaunchLog.count
+        fused = block(h, enc, temb, rope)
+        assert ops.LaunchLog.count - n0 == 6          # norm + gate twice, norm + rotary, attention
+        hooks = [m.register_forward_hook(lambda m, i, o: None) for m in (block.norm1, block.norm2.norm, block.norm_q)]
+        n0 = ops.LaunchLog.count
+        plain = block(h, enc, temb, rope)
+        assert ops.LaunchLog.count - n0 == 1
+        for x in hooks:
+            x.remove()
+    n0 = ops.LaunchLog.count
+    out = block(h, enc, temb, rope)
+    assert out[0].requires_grad and ops.LaunchLog.count - n0 == 2      # gradients of the residual path stay
+    for a, b, c in zip(fused, plain, out):            # bf16 roundings in between: a few units in the last place
+        scale = b.float().abs().max()
+        assert (a.float() - b.float()).abs().max() <= scale * 2.0 ** -5 and (c.float() - b.float()).abs().max() <= scale * 2.0 ** -5
+    rmod.destroy_redundancy_map()
