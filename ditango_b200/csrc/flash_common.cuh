@@ -120,41 +120,64 @@ __device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, 
   }
 }
 
-// Final step for 32 consecutive columns of one output row held in `orow` (un-normalised fp32 accumulators):
-// scale by w_new, blend with the state already in global memory when accumulating (w_old != 0), store as
-// fp32 or bf16.  `col` is the element offset of the 32 columns inside the row's token.
-__device__ __forceinline__ void store_row_chunk32(const FlashParams& p, int64_t tok, int64_t col, const uint32_t (&orow)[32],
-                                                  float w_new, float w_old) {
-  if (p.out_dtype == 0) {
-    float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.out) + tok * p.out_tok_stride + col);
-    if (p.accumulate && w_old != 0.f) {
+// Final step for 32 consecutive columns of a warp's 32 output rows, executed by the whole warp: lane i holds row i
+// (un-normalised fp32 accumulators `acc`) and its weights.  Scale by w_new, blend with the state already in global memory
+// when accumulating (w_old != 0), store as fp32 or bf16.  `tok0` is the token of the warp's first row, `rows` how many of
+// its rows exist, `col` the element offset of the columns inside a token; `stage` is 4 KB of shared memory of the warp.
+//
+// The rows go through shared memory so that 8 lanes write (and read) the 128 contiguous bytes of a row: a lane that
+// stores its own row touches 32 cache lines per warp instruction, half a sector of each, and the load / store unit then
+// spends a clock per line (32 x 16 instructions x 8 warps for 256 rows of 64 columns, twice that with a state to read).
+// CogVideoX ring on rank 3 of 8 3.91 -> 3.70 ms, its whole sequence 9.65 -> 9.41 ms.  The 16-byte pieces are XOR-swizzled by row, so that neither side has bank conflicts.
+__device__ __forceinline__ void store_rows32(const FlashParams& p, uint8_t* stage, int64_t tok0, int rows, int64_t col,
+                                             const uint32_t (&acc)[32], float w_new, float w_old) {
+  const int lane = threadIdx.x & 31;
+  const bool f32 = p.out_dtype == 0;
+  const int r0 = lane >> 3, piece = lane & 7;
+  float* dst = static_cast<float*>(p.out) + (tok0 + r0) * p.out_tok_stride + col + piece * 4;
+  float4 old[8];
+  if (p.accumulate) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float4 o = dst[i];
-        o.x = o.x * w_old + __uint_as_float(orow[4 * i]) * w_new;
-        o.y = o.y * w_old + __uint_as_float(orow[4 * i + 1]) * w_new;
-        o.z = o.z * w_old + __uint_as_float(orow[4 * i + 2]) * w_new;
-        o.w = o.w * w_old + __uint_as_float(orow[4 * i + 3]) * w_new;
-        dst[i] = o;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        dst[i] = make_float4(__uint_as_float(orow[4 * i]) * w_new, __uint_as_float(orow[4 * i + 1]) * w_new,
-                             __uint_as_float(orow[4 * i + 2]) * w_new, __uint_as_float(orow[4 * i + 3]) * w_new);
-    }
-  } else {
-    uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + tok * p.out_tok_stride + col);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint4 v;
-      v.x = pack_bf16x2(__uint_as_float(orow[8 * i]) * w_new, __uint_as_float(orow[8 * i + 1]) * w_new);
-      v.y = pack_bf16x2(__uint_as_float(orow[8 * i + 2]) * w_new, __uint_as_float(orow[8 * i + 3]) * w_new);
-      v.z = pack_bf16x2(__uint_as_float(orow[8 * i + 4]) * w_new, __uint_as_float(orow[8 * i + 5]) * w_new);
-      v.w = pack_bf16x2(__uint_as_float(orow[8 * i + 6]) * w_new, __uint_as_float(orow[8 * i + 7]) * w_new);
-      dst[i] = v;
+    for (int it = 0; it < 8; ++it) {
+      const float wo = __shfl_sync(0xffffffffu, w_old, it * 4 + r0);
+      old[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (it * 4 + r0 < rows && wo != 0.f) old[it] = *reinterpret_cast<const float4*>(dst + it * 4 * p.out_tok_stride);
     }
   }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    *reinterpret_cast<float4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) =
+        make_float4(__uint_as_float(acc[4 * i]) * w_new, __uint_as_float(acc[4 * i + 1]) * w_new,
+                    __uint_as_float(acc[4 * i + 2]) * w_new, __uint_as_float(acc[4 * i + 3]) * w_new);
+  __syncwarp();
+  auto staged = [&](int r, int i) { return *reinterpret_cast<const float4*>(stage + r * 128 + ((i ^ (r & 7)) << 4)); };
+  if (f32) {
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int r = it * 4 + r0;
+      float4 v = staged(r, piece);
+      if (p.accumulate) {
+        const float wo = __shfl_sync(0xffffffffu, w_old, r);
+        if (wo != 0.f) {
+          v.x = fmaf(old[it].x, wo, v.x);
+          v.y = fmaf(old[it].y, wo, v.y);
+          v.z = fmaf(old[it].z, wo, v.z);
+          v.w = fmaf(old[it].w, wo, v.w);
+        }
+      }
+      if (r < rows) *reinterpret_cast<float4*>(dst + it * 4 * p.out_tok_stride) = v;
+    }
+  } else {
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int r = it * 8 + (lane >> 2), i = (lane & 3) * 2;
+      const float4 a = staged(r, i), b = staged(r, i + 1);
+      if (r < rows)
+        *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + (tok0 + r) * p.out_tok_stride + col + i * 4) =
+            make_uint4(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w), pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
+    }
+  }
+  __syncwarp();        // the stage is written again for the next columns
 }
 
 // Weights of the final normalisation: a row whose un-normalised accumulator has row sum l_row and log-sum-exp

@@ -277,7 +277,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     const int tile = warp >> 2;
     const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t o_taddr = lane_base + C::kColO + tile * D;
     const float c = p.scale_log2;
@@ -393,25 +392,30 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // Results: the launch before this one (which may still be running if this launch overlaps it) must have
     // completed before its state is read for accumulation or its buffers are written.
     grid_dependency_wait();
+    ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
-      const int q_pos = q0 + tile * kBM + row;
-      const bool valid = q_pos < q_len;
-      const int64_t tok = static_cast<int64_t>(q_begin) + q_pos;
+      const int warp_pos = q0 + tile * kBM + quarter * 32;      // position of the warp's first row
+      const int rows = q_len - warp_pos;
+      const int64_t tok0 = static_cast<int64_t>(q_begin) + warp_pos;
       const float lse_new = (m * c + log2f(l)) * kLn2;
       float w_new = 1.f / l, w_old = 0.f;
-      if (valid) {
-        const int64_t li = lse_index(p, seg, head, q_pos, tok);
+      if (lane < rows) {
+        const int64_t li = lse_index(p, seg, head, warp_pos + lane, tok0 + lane);
         float lse_out;
         merge_weights(p.accumulate != 0, p.accumulate ? p.lse[li] : -INFINITY, lse_new, l, w_new, w_old, lse_out);
         p.lse[li] = lse_out;
       }
+      // staged in this warp's part of its Q tile, which the last S instruction has read
+      uint8_t* stage = s_q + tile * C::kTileBytes + quarter * (C::kTileBytes / 4);
+      static_assert(C::kTileBytes / 4 >= 4096, "32 rows x 128 bytes");
 #pragma unroll
       for (int q = 0; q < D / 32; ++q) {
         uint32_t orow[32];
         tmem_ld32(o_taddr + q * 32, orow);
         tmem_wait_ld();
-        if (valid) store_row_chunk32(p, tok, static_cast<int64_t>(head) * D + q * 32, orow, w_new, w_old);
+        pin32(orow);
+        if (rows > 0) store_rows32(p, stage, tok0, rows, static_cast<int64_t>(head) * D + q * 32, orow, w_new, w_old);
       }
     }
   }
