@@ -25,8 +25,8 @@
 //
 // Measured on one B200, launches alone, per step of 128 keys x 256 rows (SM clocks): the MMAs without the softmax 2250
 // at D = 128 and 1430 at D = 64, the softmax without the MMAs 2540 and 2460, both 3050 and 2680.  TFLOP/s against the
-// two kernels with 64-key tiles that this one replaced: D = 64 at 2 x 17776 tokens x 48 heads 890 (before 769), D = 128
-// at 14882 tokens x 24 heads 1274 (1170); sustained, with the board at its power cap, 1220 (1103) at 119056 tokens.
+// two kernels with 64-key tiles that this one replaced: D = 64 at 2 x 17776 tokens x 48 heads 922 (before 769), D = 128
+// at 14882 tokens x 24 heads 1286 (1170); sustained, with the board at its power cap, 1186-1220 (1103) at 119056 tokens.
 //
 // Running max is kept lazily: O is rescaled only when the max grew by more than 2^8, which bounds every
 // probability by 2^8 and keeps bf16 P exact enough; the final normalisation undoes it.
