@@ -263,9 +263,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (!ok) break;
           tc_fence_after();
           issue_pv(tile, v_stage, buf, true, kSplit / 16, kBN / 16);
-          if (NB > 2) mma_commit(&pv_done[tile]);
-          if (u >= n_units - 2) mma_commit(&o_final[tile]);
-          if (tile == 1) mma_commit(&kv_empty[v_stage]);
+          // A tile's last unit commits to o_final alone: nothing waits for its pv_done or for the ring slot, and an arrival
+          // that nothing waits for could still be under way when the CTA ends and its shared memory gets a new owner.
+          if (u >= n_units - 2) {
+            mma_commit(&o_final[tile]);
+          } else {
+            if (NB > 2) mma_commit(&pv_done[tile]);
+            if (tile == 1) mma_commit(&kv_empty[v_stage]);
+          }
           if (u + NB < n_units) ok = do_s(u + NB, buf);
           if (++buf == NB) { buf = 0; use ^= 1; }
         }

@@ -1,0 +1,117 @@
+"""The MMA issuer of the attention kernel, replayed on the CPU.
+
+The issuer's source is taken out of the kernel, compiled for the host against stubs that record every barrier wait, MMA and
+commit, and run for a few numbers of key tiles.  What it does with the tensor core cannot be seen here; the order in which it
+asks for things can."""
+import os
+import re
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "ditango_b200", "csrc")
+
+STUBS = r"""
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+%(constants)s
+%(cfg)s
+constexpr int D = %(head_dim)d;
+using C = Cfg<D>;
+constexpr int NB = C::kSBufs;
+constexpr int kRing = C::kStages;
+uint64_t q_full[2], kv_full[kRing], kv_empty[kRing], s_full[NB], p_lo[NB], p_hi[NB], pv_done[2], o_final[2];
+uint8_t s_q[1], s_kv[1];
+struct { int* status; } p;
+constexpr uint32_t idesc_bf16_f32(int, int, bool, bool) { return 0; }
+uint32_t smem_u32(const void* x) { return x == s_q ? 0u : uint32_t(kQT * C::kTileBytes); }
+uint64_t smem_desc_sw128(uint32_t addr, uint32_t, uint32_t) { return addr >> 4; }
+void event(const char* what, const uint64_t* bar, int extra) {
+#define BAR(b) if (bar >= b && bar < b + sizeof(b) / 8) std::printf("%%s %%s %%d %%d\n", what, #b, int(bar - b), extra)
+  BAR(q_full); BAR(kv_full); BAR(kv_empty); BAR(s_full); BAR(p_lo); BAR(p_hi); BAR(pv_done); BAR(o_final);
+}
+bool wait_or_abort(uint64_t* bar, uint32_t parity, int*, int) { event("wait", bar, int(parity)); return true; }
+void mma_commit(uint64_t* bar) { event("commit", bar, 0); }
+void mma_ss(uint32_t d, uint64_t, uint64_t b, uint32_t, uint32_t) { std::printf("S %%u %%llu\n", d, (unsigned long long)b); }
+void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t, uint32_t acc) {
+  std::printf("PV %%u %%u %%llu %%u\n", d, a, (unsigned long long)b, acc);
+}
+void tc_fence_after() {}
+bool elect_one() { return true; }
+int main(int, char** argv) {
+  const int k_len = std::atoi(argv[1]);
+  const int n_tiles = (k_len + kBN - 1) / kBN;
+  const int n_units = kQT * n_tiles;
+  const uint32_t tmem_base = 0;
+  (void)n_units; (void)n_tiles;
+%(issuer)s
+}
+"""
+
+
+def _block(text, start):
+    """The text from the `{` behind position `start` to its matching `}`."""
+    i = text.index("{", start)
+    depth = 0
+    for j in range(i, len(text)):
+        depth += (text[j] == "{") - (text[j] == "}")
+        if depth == 0:
+            return text[i:j + 1]
+    raise AssertionError("unbalanced braces")
+
+
+@pytest.fixture(scope="module")
+def replay(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no host compiler")
+    kernel = open(os.path.join(CSRC, "flash_fwd_sm100.cu")).read()
+    common = open(os.path.join(CSRC, "flash_common.cuh")).read()
+    constants = "\n".join(re.findall(r"^constexpr int k\w+ = [^;]*;", common, re.M) + re.findall(r"^constexpr int k\w+ = [^;]*;", kernel, re.M))
+    cfg = "template <int D>\nstruct Cfg " + _block(kernel, kernel.index("struct Cfg")) + ";"
+    issuer = _block(kernel, kernel.index("if (elect_one())", kernel.index("- MMA issuer")))
+    built = {}
+    for head_dim in (64, 128):
+        d = tmp_path_factory.mktemp("issuer")
+        src, exe = str(d / "issuer.cpp"), str(d / "issuer")
+        with open(src, "w") as f:
+            f.write(STUBS % dict(constants=constants, cfg=cfg, issuer=issuer, head_dim=head_dim))
+        r = subprocess.run([gxx, "-std=c++17", "-O0", "-w", src, "-o", exe], capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr
+        built[head_dim] = exe
+
+    def run(head_dim, k_len):
+        r = subprocess.run([built[head_dim], str(k_len)], capture_output=True, text=True)
+        assert r.returncode == 0
+        return [line.split() for line in r.stdout.splitlines()]
+    return run
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("tiles", [1, 2, 3, 4, 7, 12])
+def test_no_arrival_is_left_behind_the_one_the_epilogue_waits_for(replay, head_dim, tiles):
+    """Threads leave the CTA once both o_final barriers have completed.  Every other commit therefore has an MMA behind it
+    that the last o_final commit covers, and none follows that."""
+    ev = replay(head_dim, 128 * tiles)
+    finals = [i for i, e in enumerate(ev) if e[:2] == ["commit", "o_final"]]
+    assert [ev[i][2] for i in finals] == ["0", "1"] and finals[-1] == len(ev) - 1
+    last_mma = max(i for i, e in enumerate(ev) if e[0] in ("S", "PV"))
+    assert all(i < last_mma for i, e in enumerate(ev) if e[0] == "commit" and e[1] != "o_final")
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("tiles", [1, 2, 3, 4, 7, 12])
+def test_every_wait_has_its_arrival(replay, head_dim, tiles):
+    """The waits of the softmax warps and of the loads, counted against the issuer's commits."""
+    ev = replay(head_dim, 128 * tiles)
+    count = lambda name: sum(e[:2] == ["commit", name] for e in ev)
+    stages = max(int(e[2]) for e in ev if e[1:2] == ["kv_full"]) + 1
+    assert count("s_full") == 2 * tiles
+    assert count("kv_empty") >= 2 * tiles - stages           # a slot is waited for before its next load
+    if head_dim == 64:
+        assert count("pv_done") >= 2 * (tiles - 1)           # a rescale in tile j waits for PV of tile j - 1
+    loads = [(int(e[2]), int(e[3])) for e in ev if e[:2] == ["wait", "kv_full"]]
+    ring = {64: 10, 128: 5}[head_dim]
+    assert loads == [(i % ring, (i // ring) & 1) for i in range(2 * tiles)]
