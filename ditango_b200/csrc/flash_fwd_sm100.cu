@@ -116,7 +116,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     k_len = p.seqlen_k;
   }
   const int q0 = blockIdx.x * (kQT * kBM);
-  if (q0 >= q_len) return;
+  if (q0 >= q_len) {
+    // (see the tear-down; a grid whose sequences are all empty has no CTA that gets that far)
+    if (blockIdx.x == 0) grid_dependency_wait();
+    return;
+  }
   const int n_tiles = (k_len + kBN - 1) / kBN;
   if (n_tiles <= 0) {
     grid_dependency_wait();      // (also when nothing is written: a grid must not complete before the one it overlaps)

@@ -115,3 +115,19 @@ def test_every_wait_has_its_arrival(replay, head_dim, tiles):
     loads = [(int(e[2]), int(e[3])) for e in ev if e[:2] == ["wait", "kv_full"]]
     ring = {64: 10, 128: 5}[head_dim]
     assert loads == [(i % ring, (i // ring) & 1) for i in range(2 * tiles)]
+
+
+def test_every_way_out_of_the_kernel_waits_for_the_launch_it_may_overlap():
+    """A launch that overlaps this one waits for this grid only, so no grid may complete before the one it overlaps: each
+    early return waits first (of the blocks past a sequence's end the first of an empty sequence does: a grid in which every
+    block returns there has only empty sequences)."""
+    kernel = open(os.path.join(CSRC, "flash_fwd_sm100.cu")).read()
+    body = _block(kernel, kernel.index("const FlashParams p) {\n  using C"))
+    returns = [m.start() for m in re.finditer(r"\breturn;", body)]
+    assert len(returns) == 2
+    for at in returns:
+        scope = body[body.rindex("{", 0, at):at]
+        assert "grid_dependency_wait();" in scope, scope
+    assert "if (blockIdx.x == 0) grid_dependency_wait();" in body[:returns[0]]
+    tail = body[body.rindex("tear-down"):]
+    assert tail.index("grid_dependency_wait();") < tail.index("__syncthreads();")

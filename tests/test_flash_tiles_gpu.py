@@ -71,3 +71,25 @@ def test_a_nan_key_reaches_every_row(D, key):
     o, l = ops.flash_partial(q, k, v)
     assert torch.isnan(o).all() and torch.isnan(l).all()
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_launch_of_empty_sequences_does_not_break_a_chain_of_overlapping_ones(D):
+    """Three overlapping launches on one state, the middle one without a single query row: same bits as separate launches."""
+    from ditango_b200 import ops
+    q, k, v = (x.flatten(0, 1) for x in _qkv(1, 3000, 3000, 6, D))
+    full = torch.tensor([0, 3000], dtype=torch.int32, device="cuda")
+    none = torch.zeros(2, dtype=torch.int32, device="cuda")
+
+    def chain(overlap):
+        o, l = ops.flash_partial(q, k, v, cu_seqlens_q=full, cu_seqlens_k=full)
+        for cu in (none, full):
+            ops.flash_partial(q, v, k, cu_seqlens_q=cu, cu_seqlens_k=full, out=o, lse=l, accumulate=True, overlap_previous=overlap)
+        return o, l
+
+    want = chain(False)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        got = chain(True)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert ops.read_status() == 0
