@@ -67,14 +67,6 @@ struct Cfg {
   static_assert(kSmemBytes <= 232448, "shared memory");
 };
 
-__device__ __forceinline__ void pin32(uint32_t* r) {
-#pragma unroll
-  for (int i = 0; i < 32; i += 8)
-    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]),
-                      "+r"(r[i + 7]));
-}
-
-
 }  // namespace
 
 template <int D>
@@ -303,9 +295,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       uint32_t sr[kBN];
       tmem_ld32(s_taddr, sr);
       tmem_ld32(s_taddr + 32, sr + 32);
-      tmem_wait_ld();
-      pin32(sr);
-      pin32(sr + 32);
+      tmem_wait_ld<64>(sr);
       tmem_ld32(s_taddr + 64, sr + 64);      // in flight while the first half is scanned
       tmem_ld32(s_taddr + 96, sr + 96);
       const bool ragged = (j == n_tiles - 1) && (k_len & (kBN - 1)) != 0;
@@ -326,9 +316,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       };
       scan(0);
-      tmem_wait_ld();
-      pin32(sr + 64);
-      pin32(sr + 96);
+      tmem_wait_ld<64>(sr + 64);
       if (ragged) {
 #pragma unroll
         for (int i = 64; i < kBN; ++i)
@@ -353,7 +341,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           for (int q = 0; q < D / 16; ++q) {
             uint32_t orow[16];
             tmem_ld16(o_taddr + q * 16, orow);
-            tmem_wait_ld();
+            tmem_wait_ld<16>(orow);
 #pragma unroll
             for (int i = 0; i < 16; ++i) orow[i] = __float_as_uint(__uint_as_float(orow[i]) * f);
             tmem_st16(o_taddr + q * 16, orow);
@@ -422,8 +410,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       for (int q = 0; q < D / 32; ++q) {
         uint32_t orow[32];
         tmem_ld32(o_taddr + q * 32, orow);
-        tmem_wait_ld();
-        pin32(orow);
+        tmem_wait_ld<32>(orow);
         if (rows > 0) store_rows32(p, stage, tok0, rows, static_cast<int64_t>(head) * D + q * 32, orow, w_new, w_old);
       }
     }

@@ -69,7 +69,18 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Waits for this thread's tcgen05.ld and makes the N registers `r` they were given results of the wait: without that
+// nothing orders arithmetic on them behind it (a "memory" clobber does not concern registers).  Registers of loads that are
+// to stay in flight are left out, and so need a wait of their own.
+template <int N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t* r) {
+  static_assert(N % 8 == 0, "registers are pinned by eights");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < N; i += 8)
+    asm volatile("" : "+r"(r[i]), "+r"(r[i + 1]), "+r"(r[i + 2]), "+r"(r[i + 3]), "+r"(r[i + 4]), "+r"(r[i + 5]), "+r"(r[i + 6]),
+                      "+r"(r[i + 7]));
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Lane L of the warp reads 32 consecutive 32-bit columns of TMEM lane (taddr.lane + L).

@@ -131,3 +131,29 @@ def test_every_way_out_of_the_kernel_waits_for_the_launch_it_may_overlap():
     assert "if (blockIdx.x == 0) grid_dependency_wait();" in body[:returns[0]]
     tail = body[body.rindex("tear-down"):]
     assert tail.index("grid_dependency_wait();") < tail.index("__syncthreads();")
+
+
+def test_every_tensor_memory_load_is_waited_for_with_its_registers():
+    """tcgen05.wait::ld orders arithmetic on loaded registers only if they are operands of the wait."""
+    kernel = open(os.path.join(CSRC, "flash_fwd_sm100.cu")).read()
+    sources = {name: open(os.path.join(CSRC, name)).read() for name in os.listdir(CSRC) if name.endswith((".cu", ".cuh"))}
+    assert sum(text.count('"tcgen05.wait::ld') for text in sources.values()) == 1      # one helper, which takes the registers
+    helper = _block(sources["ptx_sm100.cuh"], sources["ptx_sm100.cuh"].index("void tmem_wait_ld(uint32_t* r)"))
+    assert '"+r"(r[i])' in helper
+
+    def where(arg):
+        name, _, offset = arg.partition("+")
+        return name.strip(), int(offset or 0)
+
+    asked, events = {}, re.finditer(r"tmem_ld(\d+)\([^;]*, ([\w +]+)\);|tmem_wait_ld<(\d+)>\(([\w +]+)\);|tmem_wait_ld", kernel)
+    for m in events:
+        if m.group(1):
+            name, at = where(m.group(2))
+            asked.setdefault(name, set()).update(range(at, at + int(m.group(1))))
+        else:
+            assert m.group(3), "a wait without registers"
+            name, at = where(m.group(4))
+            covered = set(range(at, at + int(m.group(3))))
+            assert covered <= asked[name]
+            asked[name] -= covered
+    assert asked and not any(asked.values())
