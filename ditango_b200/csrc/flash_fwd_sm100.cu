@@ -57,8 +57,8 @@ struct Cfg {
   static constexpr int kKvTileBytes = kBN * D * 2;      // one K or V tile
   static constexpr int kStages = (D == 128) ? 5 : 10;
   static constexpr int kSBufs = (512 - kQT * D) / kBN;
-  // barriers: q_full[2], kv_full[S], kv_empty[S], s_full[NB], p_lo[NB], p_hi[NB], pv_done[2], o_final[2]
-  static constexpr int kBars = 2 + 2 * kStages + 3 * kSBufs + 2 + 2;
+  // barriers: q_full[2], kv_full[S], kv_empty[S], s_full[NB], p_lo[NB], p_hi[NB], pv_done[2], o_final[2], v_tail[1]
+  static constexpr int kBars = 2 + 2 * kStages + 3 * kSBufs + 2 + 2 + 1;
   static constexpr int kSmemBytes = 1024 + kQT * kTileBytes + kStages * kKvTileBytes + kBars * 8 + 16;
   static constexpr uint32_t kTmemCols = 512;
   static constexpr uint32_t kColS = 0;                    // + buffer * 128
@@ -88,6 +88,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint64_t* p_hi = p_lo + NB;                 // [buffer]: the rest of P(u) written
   uint64_t* pv_done = p_hi + NB;              // [tile]: PV(u) has completed
   uint64_t* o_final = pv_done + 2;            // [tile]: the last PV of the tile has completed
+  uint64_t* v_tail = o_final + 2;             // the foreign rows of the last V tile's last K step have been cleared
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kBars);
 
   const int warp = threadIdx.x >> 5;
@@ -128,6 +129,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_init(&pv_done[i], 1);
       mbar_init(&o_final[i], 1);
     }
+    mbar_init(v_tail, 1);
     for (int i = 0; i < C::kStages; ++i) {
       mbar_init(&kv_full[i], 1);
       mbar_init(&kv_empty[i], 1);
@@ -154,10 +156,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   if (warp >= kTmaWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+    // The last key tile holds `tail` keys of this sequence; the rows behind them belong to whatever follows it in memory (or
+    // are TMA's zeros past the end of the tensor).  Their scores are masked, but a weight of 0 does not keep an infinity or
+    // a NaN of their V rows out of the product: PV of the last tile runs the K steps of 16 keys that hold a key, and the
+    // foreign rows of the last of these are cleared in shared memory first.
+    const int tail = k_len - (n_tiles - 1) * kBN;
+    const int tail_steps = (tail + 15) >> 4;
     if (aborted || warp > kMmaWarp) {
       // fall through to the tear-down
     } else if (warp == kTmaWarp) {
       // ------------------------------------------------------------ TMA producer
+      bool live = true;
       if (elect_one()) {
         prefetch_tmap(&tm_q);
         prefetch_tmap(&tm_k);
@@ -180,7 +189,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         };
         // in the order in which the issuer consumes them
         load_q(0);
-        bool live = load_kv(&tm_k, 0);
+        live = load_kv(&tm_k, 0);
         load_q(1);
         if (NB > 2 && live && n_tiles > 1) live = load_kv(&tm_k, 1);
         for (int u = 0; live && u < n_units; ++u) {
@@ -190,6 +199,24 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       }
       __syncwarp();
+      if ((tail & 15) != 0 && __all_sync(0xffffffffu, live)) {
+        const int it = 2 * n_tiles - 1;                 // V of the last tile is the last load
+        const int stage = it % C::kStages;
+        const bool landed = wait_or_abort(&kv_full[stage], (it / C::kStages) & 1, p.status, 12);
+        if (__all_sync(0xffffffffu, landed)) {
+          // whole rows of 128 bytes: the swizzle moves 16-byte pieces inside a row only
+#pragma unroll 1
+          for (int s = 0; s < C::kSlabs; ++s) {
+            uint8_t* first = s_kv + stage * C::kKvTileBytes + s * kSlabBytes + tail * 128;
+#pragma unroll 1
+            for (int i = lane; i < (16 * tail_steps - tail) * 8; i += 32)
+              *reinterpret_cast<uint4*>(first + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          fence_proxy_async_smem();                     // the MMA reads shared memory through the asynchronous proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(v_tail);
+        }
+      }
     } else {
       // ------------------------------------------------------------ MMA issuer
       if (elect_one()) {
@@ -213,14 +240,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             mma_ss(d, a0 + off, b0 + off, idesc_qk, k16 > 0);
           }
         };
-        // O_tile (+)= P V over the keys [16 k0, 16 k1) of the tile; P (bf16 pairs) at the start of S buffer `buf`
-        auto issue_pv = [&](int tile, int stage, int buf, bool acc, int k0, int k1) {
+        // O_tile (+)= P V over the K steps [k0, k1) of 16 keys, as far as the tile has `steps`; P (bf16 pairs) at the start
+        // of S buffer `buf`
+        auto issue_pv = [&](int tile, int stage, int buf, bool acc, int k0, int k1, int steps) {
           const uint64_t b0 = v_desc + static_cast<uint32_t>(stage * (C::kKvTileBytes >> 4));
           const uint32_t d = tmem_base + C::kColO + tile * D;
           const uint32_t a = tmem_base + C::kColS + buf * kBN;
 #pragma unroll
           for (int kk = k0; kk < k1; ++kk)
-            mma_ts(d, a + kk * 8, b0 + (kk * 2048 >> 4), idesc_pv, (acc || kk > 0) ? 1u : 0u);
+            if (kk < steps) mma_ts(d, a + kk * 8, b0 + (kk * 2048 >> 4), idesc_pv, (acc || kk > 0) ? 1u : 0u);
         };
         int stage = 0;             // next ring slot to consume
         uint32_t round = 0;        // its parity
@@ -248,26 +276,39 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         for (int u = 0; ok && u < NB && u < n_units; ++u) ok = do_s(u, u);
         int buf = 0;
         uint32_t use = 0;          // parity of the buffer's barriers
-        for (int u = 0; ok && u < n_units; ++u) {
+        int u = 0;
+        for (; ok && u < n_units - 2; ++u) {
           const int tile = u & 1;
           if (tile == 0 && !next_kv(v_stage, 23)) { ok = false; break; }
           ok = wait_or_abort(&p_lo[buf], use, p.status, 24 + tile);
           if (!ok) break;
           tc_fence_after();
-          issue_pv(tile, v_stage, buf, u > 1, 0, kSplit / 16);
+          issue_pv(tile, v_stage, buf, u > 1, 0, kSplit / 16, kBN / 16);
           ok = wait_or_abort(&p_hi[buf], use, p.status, 26 + tile);
           if (!ok) break;
           tc_fence_after();
-          issue_pv(tile, v_stage, buf, true, kSplit / 16, kBN / 16);
-          // A tile's last unit commits to o_final alone: nothing waits for its pv_done or for the ring slot, and an arrival
-          // that nothing waits for could still be under way when the CTA ends and its shared memory gets a new owner.
-          if (u >= n_units - 2) {
-            mma_commit(&o_final[tile]);
-          } else {
-            if (NB > 2) mma_commit(&pv_done[tile]);
-            if (tile == 1) mma_commit(&kv_empty[v_stage]);
-          }
+          issue_pv(tile, v_stage, buf, true, kSplit / 16, kBN / 16, kBN / 16);
+          if (NB > 2) mma_commit(&pv_done[tile]);
+          if (tile == 1) mma_commit(&kv_empty[v_stage]);
           if (u + NB < n_units) ok = do_s(u + NB, buf);
+          if (++buf == NB) { buf = 0; use ^= 1; }
+        }
+        // The last key tile, behind the loop so that the loop's PV has no limit to test (with one test per MMA in the loop the
+        // kernel was 1-2 % slower, like this 0.3 %).  It commits to o_final alone: nothing waits for its pv_done or for the ring
+        // slot, and an arrival that nothing waits for could still be under way when the CTA ends and its shared memory gets
+        // a new owner.
+        ok = ok && next_kv(v_stage, 23) && ((tail & 15) == 0 || wait_or_abort(v_tail, 0, p.status, 28));
+#pragma unroll 1
+        for (int tile = 0; ok && tile < kQT; ++tile) {
+          ok = wait_or_abort(&p_lo[buf], use, p.status, 24 + tile);
+          if (!ok) break;
+          tc_fence_after();
+          issue_pv(tile, v_stage, buf, n_tiles > 1, 0, kSplit / 16, tail_steps);
+          ok = wait_or_abort(&p_hi[buf], use, p.status, 26 + tile);
+          if (!ok) break;
+          tc_fence_after();
+          issue_pv(tile, v_stage, buf, true, kSplit / 16, kBN / 16, tail_steps);
+          mma_commit(&o_final[tile]);
           if (++buf == NB) { buf = 0; use ^= 1; }
         }
       }

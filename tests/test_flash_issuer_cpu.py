@@ -22,7 +22,7 @@ constexpr int D = %(head_dim)d;
 using C = Cfg<D>;
 constexpr int NB = C::kSBufs;
 constexpr int kRing = C::kStages;
-uint64_t q_full[2], kv_full[kRing], kv_empty[kRing], s_full[NB], p_lo[NB], p_hi[NB], pv_done[2], o_final[2];
+uint64_t q_full[2], kv_full[kRing], kv_empty[kRing], s_full[NB], p_lo[NB], p_hi[NB], pv_done[2], o_final[2], v_tail[1];
 uint8_t s_q[1], s_kv[1];
 struct { int* status; } p;
 constexpr uint32_t idesc_bf16_f32(int, int, bool, bool) { return 0; }
@@ -30,7 +30,7 @@ uint32_t smem_u32(const void* x) { return x == s_q ? 0u : uint32_t(kQT * C::kTil
 uint64_t smem_desc_sw128(uint32_t addr, uint32_t, uint32_t) { return addr >> 4; }
 void event(const char* what, const uint64_t* bar, int extra) {
 #define BAR(b) if (bar >= b && bar < b + sizeof(b) / 8) std::printf("%%s %%s %%d %%d\n", what, #b, int(bar - b), extra)
-  BAR(q_full); BAR(kv_full); BAR(kv_empty); BAR(s_full); BAR(p_lo); BAR(p_hi); BAR(pv_done); BAR(o_final);
+  BAR(q_full); BAR(kv_full); BAR(kv_empty); BAR(s_full); BAR(p_lo); BAR(p_hi); BAR(pv_done); BAR(o_final); BAR(v_tail);
 }
 bool wait_or_abort(uint64_t* bar, uint32_t parity, int*, int) { event("wait", bar, int(parity)); return true; }
 void mma_commit(uint64_t* bar) { event("commit", bar, 0); }
@@ -44,8 +44,9 @@ int main(int, char** argv) {
   const int k_len = std::atoi(argv[1]);
   const int n_tiles = (k_len + kBN - 1) / kBN;
   const int n_units = kQT * n_tiles;
+  const int tail = k_len - (n_tiles - 1) * kBN;
+  const int tail_steps = (tail + 15) >> 4;
   const uint32_t tmem_base = 0;
-  (void)n_units; (void)n_tiles;
 %(issuer)s
 }
 """
@@ -157,3 +158,22 @@ def test_every_tensor_memory_load_is_waited_for_with_its_registers():
             assert covered <= asked[name]
             asked[name] -= covered
     assert asked and not any(asked.values())
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("k_len", [1, 15, 16, 17, 63, 64, 65, 112, 113, 127, 128, 129, 192, 255, 384, 391])
+def test_pv_of_the_last_tile_stays_within_the_sequence(replay, head_dim, k_len):
+    """PV covers all 128 keys of every tile but the last, there the steps of 16 keys that hold one; where the last step also
+    holds foreign rows, the wait for their clearing is in front of it."""
+    ev = replay(head_dim, k_len)
+    tiles = -(-k_len // 128)
+    per_tile = [8] * (tiles - 1) + [-(-(k_len - 128 * (tiles - 1)) // 16)]
+    pv = [i for i, e in enumerate(ev) if e[0] == "PV"]
+    assert len(pv) == 2 * sum(per_tile)
+    last = pv[-2 * per_tile[-1]:]
+    waits = [i for i, e in enumerate(ev) if e[:2] == ["wait", "v_tail"]]
+    assert len(waits) == (1 if k_len % 16 else 0) and all(i < last[0] for i in waits)
+    slot = lambda i: int(ev[i][3])
+    for q_tile in range(2):                       # steps of one Q tile: K steps of 16 rows of 128 bytes, in units of 16 bytes
+        mine = last[q_tile * per_tile[-1]:(q_tile + 1) * per_tile[-1]]
+        assert [slot(i) - slot(mine[0]) for i in mine] == [128 * s for s in range(per_tile[-1])]

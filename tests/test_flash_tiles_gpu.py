@@ -93,3 +93,26 @@ def test_a_launch_of_empty_sequences_does_not_break_a_chain_of_overlapping_ones(
         got = chain(True)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sk", [1, 15, 16, 17, 63, 64, 65, 100, 127, 128, 129, 192, 255, 270])
+def test_a_neighbour_that_is_not_finite_stays_outside(D, Sk):
+    """The last key tile of a sequence reads rows of whatever lies behind it: the next batch item, the next packed segment,
+    rows past the last offset.  Infinities and NaN there must not change a bit of the result."""
+    from ditango_b200 import ops
+    Sq = 200
+    q, k, v = _qkv(2, Sq, Sk, 2, D)
+    clean = ops.flash_partial(q, k, v)
+    cu_q, cu_k = (torch.tensor([0, n, 2 * n], dtype=torch.int32, device="cuda") for n in (Sq, Sk))
+    for bad in (float("nan"), float("inf")):
+        kb, vb = k.clone(), v.clone()
+        kb[1], vb[1] = bad, bad
+        o, l = ops.flash_partial(q, kb, vb)                                          # dense, behind batch item 0
+        assert torch.equal(o[0], clean[0][0]) and torch.equal(l[0], clean[1][0]) and torch.isnan(o[1]).all()
+        qp, kp, vp = (x.flatten(0, 1) for x in (q, kb, vb))
+        o, l = ops.flash_partial(qp, kp, vp, cu_seqlens_q=cu_q, cu_seqlens_k=cu_k)   # packed, behind segment 0
+        assert torch.equal(o[:Sq], clean[0][0]) and torch.equal(l[:, :Sq], clean[1][0])
+        o, l = ops.flash_partial(qp, kp, vp, cu_seqlens_q=cu_q[:2].contiguous(), cu_seqlens_k=cu_k[:2].contiguous())
+        assert torch.equal(o[:Sq], clean[0][0]) and torch.equal(l[:, :Sq], clean[1][0])
+    assert ops.read_status() == 0
