@@ -109,6 +109,22 @@ def norm_and_rotate(q, k, norm_q, norm_k, cos, sin, text_len: int) -> Tuple[torc
     return q.contiguous(), k.contiguous()
 
 
+def _plain_modulation(h: torch.Tensor, mod: torch.Tensor) -> bool:
+    """Whether the kernels can take `mod`: one bf16 row per sequence of h.  (A row that broadcasts over the batch, another
+    dtype or layout -- what a hook on, or a replacement of, the projection may return -- stays with the separate operations.)"""
+    return tuple(mod.shape) == (h.shape[0], 6 * h.shape[-1]) and _plain_bf16(h.device, mod)
+
+
+def gated_residual(h, enc, a, mod) -> Tuple[torch.Tensor, torch.Tensor]:
+    """(h, enc) + gate * (their parts of the joint tensor a [B, text + video, dim], text first), gates from the modulation.
+    For streams that LayerNormZero.fuses; one kernel where `a` and `mod` allow it."""
+    text_len = enc.shape[1]
+    if _plain_modulation(h, mod) and tuple(a.shape) == (h.shape[0], text_len + h.shape[1], h.shape[2]) and _plain_bf16(h.device, a):
+        return _engine.gate_add(h, enc, a, mod)
+    _, _, gate, _, _, e_gate = mod.chunk(6, dim=1)
+    return h + gate[:, None] * a[:, text_len:], enc + e_gate[:, None] * a[:, :text_len]
+
+
 class LayerNormZero(nn.Module):
     def __init__(self, time_dim: int, dim: int):
         super().__init__()
@@ -122,16 +138,21 @@ class LayerNormZero(nn.Module):
         return (h.is_cuda and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda") and
                 dim % 256 == 0 and dim <= _engine.MOD_MAX_DIM and h.numel() > 0 and enc.numel() > 0 and
                 _plain_bf16(h.device, h, enc) and
-                self.linear.weight.dtype == torch.bfloat16 and
                 _unobserved(self, LayerNormZero) and _plain_norm(self.norm, dim, h.device))
 
     def joint(self, h, enc, temb):
-        """([B, text + video, dim] normalised and modulated, text first; the modulation, whose gates ops.gate_add takes)."""
-        mod = self.linear(F.silu(temb)).contiguous()
-        return _engine.ln_modulate(h, enc, self.norm.weight, self.norm.bias, self.norm.eps, mod), mod
+        """([B, text + video, dim] normalised and modulated, text first; the modulation, whose gates gated_residual takes)."""
+        mod = self.linear(F.silu(temb))
+        if _plain_modulation(h, mod):
+            return _engine.ln_modulate(h, enc, self.norm.weight, self.norm.bias, self.norm.eps, mod), mod
+        nh, nenc, _, _ = self.modulate(h, enc, mod)
+        return torch.cat([nenc, nh], dim=1), mod
 
     def forward(self, h, enc, temb):
-        shift, scale, gate, e_shift, e_scale, e_gate = self.linear(F.silu(temb)).chunk(6, dim=1)
+        return self.modulate(h, enc, self.linear(F.silu(temb)))
+
+    def modulate(self, h, enc, mod):
+        shift, scale, gate, e_shift, e_scale, e_gate = mod.chunk(6, dim=1)
         h = self.norm(h) * (1 + scale)[:, None] + shift[:, None]
         enc = self.norm(enc) * (1 + e_scale)[:, None] + e_shift[:, None]
         return h, enc, gate[:, None], e_gate[:, None]
@@ -187,7 +208,7 @@ class DiTBlock(nn.Module):
         text_len = enc.shape[1]
         if self.mode != "ulysses" and self.norm1.fuses(h, enc):
             x, mod = self.norm1.joint(h, enc, temb)
-            h, enc = _engine.gate_add(h, enc, self._attend_joint(x, text_len, rope), mod)
+            h, enc = gated_residual(h, enc, self._attend_joint(x, text_len, rope), mod)
         else:
             nh, nenc, gate, e_gate = self.norm1(h, enc, temb)
             a_h, a_enc = self._attend(nh, nenc, rope)
@@ -195,7 +216,7 @@ class DiTBlock(nn.Module):
             enc = enc + e_gate * a_enc
         if self.norm2.fuses(h, enc):
             x, mod = self.norm2.joint(h, enc, temb)
-            return _engine.gate_add(h, enc, self._feed_forward(x), mod)
+            return gated_residual(h, enc, self._feed_forward(x), mod)
         nh, nenc, gate, e_gate = self.norm2(h, enc, temb)
         ff = self._feed_forward(torch.cat([nenc, nh], dim=1))
         return h + gate * ff[:, text_len:], enc + e_gate * ff[:, :text_len]

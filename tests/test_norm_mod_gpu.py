@@ -67,3 +67,72 @@ def test_block_takes_the_fused_path_only_where_nothing_observes_it():
         scale = b.float().abs().max()
         assert (a.float() - b.float()).abs().max() <= scale * 2.0 ** -5 and (c.float() - b.float()).abs().max() <= scale * 2.0 ** -5
     rmod.destroy_redundancy_map()
+
+
+@pytest.fixture
+def block_inputs():
+    """A bf16 block of four heads, its streams (batch 2), a timestep embedding and unit rotary tables."""
+    from ditango_b200.core import redundancy_map as rmod
+    from ditango_b200.core.config import init_config
+    from ditango_b200.core.group_coordinate import SingleRankGroup
+    from ditango_b200.executor.cogvideox_dit import DiTBlock, DiTConfig
+    from ditango_b200.utils import update_timestep
+    cfg = init_config(None, make_output_dir=False)
+    cfg.num_layers, cfg.num_inference_steps = 1, 1
+    rmod.destroy_redundancy_map()
+    rmod.init_redundancy_map(cfg, world_size=1)
+    update_timestep(0)
+    torch.manual_seed(1)
+    dc = DiTConfig(num_layers=1, num_heads=4, frames=1, height=8, width=8, text_len=5)
+    block = DiTBlock(dc, 0, SingleRankGroup(torch.device("cuda", 0)), "ditango").cuda().to(torch.bfloat16)
+    h, enc, temb = (torch.randn(s, device="cuda").to(torch.bfloat16) for s in ((2, 16, 256), (2, 5, 256), (2, 512)))
+    yield block, h, enc, temb, (torch.ones(16, 64, device="cuda"), torch.zeros(16, 64, device="cuda"))
+    rmod.destroy_redundancy_map()
+
+
+def _general(block, *args):
+    """The block with its separate operations: a hook on the layers that the kernels would stand in for."""
+    hooks = [m.register_forward_hook(lambda m, i, o: None) for m in (block.norm1, block.norm2, block.norm_q)]
+    try:
+        return block(*args)
+    finally:
+        for x in hooks:
+            x.remove()
+
+
+def _close(got, want):
+    for a, b in zip(got, want):                       # bf16 roundings in between, as above
+        assert a.dtype == b.dtype and a.shape == b.shape
+        assert (a.float() - b.float()).abs().max() <= b.float().abs().max() * 2.0 ** -5
+
+
+@torch.no_grad()
+def test_one_timestep_for_the_whole_batch(block_inputs):
+    block, h, enc, temb, rope = block_inputs
+    _close(block(h, enc, temb[:1], rope), _general(block, h, enc, temb[:1], rope))
+    _close(block(h, enc, temb[:1], rope), block(h, enc, temb[:1].expand(2, -1), rope))
+
+
+def _strided(m, i, o):
+    return torch.stack([o, o], dim=-1)[..., 0]
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("where,hook", [
+    ("to_out", _strided), ("ff_out", _strided), ("norm1.linear", _strided), ("norm2.linear", _strided),
+    ("ff_out", lambda m, i, o: o.float()), ("ff_out", lambda m, i, o: o[:, :, :1]), ("to_out", lambda m, i, o: o[:1])])
+def test_a_projection_whose_output_a_hook_replaces(block_inputs, where, hook):
+    block, *args = block_inputs
+    handle = block.get_submodule(where).register_forward_hook(hook)
+    _close(block(*args), _general(block, *args))
+    handle.remove()
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("norm", ["norm1", "norm2"])
+def test_a_modulation_without_a_weight_of_its_own(block_inputs, norm):
+    block, *args = block_inputs
+    plain = block(*args)
+    layer = getattr(block, norm)
+    layer.linear = torch.nn.Sequential(layer.linear)
+    _close(block(*args), plain)
