@@ -17,6 +17,7 @@ from typing import Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from ..baseline.ulysses import heads_to_sequence, sequence_to_heads
 from ..core.attention import proAttention
@@ -80,16 +81,30 @@ def _unobserved(m: nn.Module, kind: type) -> bool:
                  mod._global_backward_pre_hooks))
 
 
+def _addressable(*tensors: torch.Tensor) -> bool:
+    """Whether a kernel that is given addresses sees all there is to `tensors`: values in memory of their own (no subclass,
+    nothing that torch.func wraps) and no forward-mode tangent, which it would drop.  Alignment: 16 bytes."""
+    for x in tensors:
+        if type(x) not in (torch.Tensor, nn.Parameter):
+            return False
+        try:
+            address = x.data_ptr()
+        except RuntimeError:
+            return False
+        if address == 0 or address % 16 or forward_ad.unpack_dual(x).tangent is not None:
+            return False
+    return True
+
+
 def _plain_norm(norm: nn.Module, dim: int, device: torch.device) -> bool:
     """True for a bf16 LayerNorm over the last `dim` channels on `device` that a kernel may stand in for."""
     return (_unobserved(norm, nn.LayerNorm) and tuple(norm.normalized_shape) == (dim,) and
             norm.weight is not None and norm.bias is not None and norm.weight.dtype == norm.bias.dtype == torch.bfloat16 and
-            norm.weight.device == norm.bias.device == device and
-            norm.weight.data_ptr() % 16 == 0 and norm.bias.data_ptr() % 16 == 0)
+            norm.weight.device == norm.bias.device == device and _addressable(norm.weight, norm.bias))
 
 
 def _plain_bf16(device: torch.device, *tensors: torch.Tensor) -> bool:
-    return all(x.dtype == torch.bfloat16 and x.device == device and x.is_contiguous() and x.data_ptr() % 16 == 0 for x in tensors)
+    return all(x.dtype == torch.bfloat16 and x.device == device and x.is_contiguous() for x in tensors) and _addressable(*tensors)
 
 
 def norm_and_rotate(q, k, norm_q, norm_k, cos, sin, text_len: int) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -99,7 +114,7 @@ def norm_and_rotate(q, k, norm_q, norm_k, cos, sin, text_len: int) -> Tuple[torc
     if (q.is_cuda and D in (64, 128) and q.shape == k.shape and _plain_bf16(q.device, q, k) and
             _plain_norm(norm_q, D, q.device) and _plain_norm(norm_k, D, q.device) and
             all(x.dtype == torch.float32 and x.shape == (q.shape[1] - text_len, D) and x.is_contiguous() and
-                x.device == q.device and x.data_ptr() % 16 == 0 for x in (cos, sin)) and
+                x.device == q.device and (x.numel() == 0 or _addressable(x)) for x in (cos, sin)) and
             not torch.is_autocast_enabled("cuda")):
         return _engine.norm_rope(q, k, (norm_q.weight, norm_q.bias, norm_q.eps), (norm_k.weight, norm_k.bias, norm_k.eps),
                                  cos, sin, text_len)
@@ -136,7 +151,7 @@ class LayerNormZero(nn.Module):
         none), and no hook on the modules whose calls it skips."""
         dim = h.shape[-1]
         return (h.is_cuda and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda") and
-                dim % 256 == 0 and dim <= _engine.MOD_MAX_DIM and h.numel() > 0 and enc.numel() > 0 and
+                dim % 256 == 0 and dim <= _engine.MOD_MAX_DIM and
                 _plain_bf16(h.device, h, enc) and
                 _unobserved(self, LayerNormZero) and _plain_norm(self.norm, dim, h.device))
 

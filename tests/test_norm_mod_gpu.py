@@ -136,3 +136,44 @@ def test_a_modulation_without_a_weight_of_its_own(block_inputs, norm):
     layer = getattr(block, norm)
     layer.linear = torch.nn.Sequential(layer.linear)
     _close(block(*args), plain)
+
+
+@torch.no_grad()
+@pytest.mark.parametrize("which", range(3))
+def test_forward_mode_tangents_are_not_dropped(block_inputs, which):
+    """A tangent on the video stream, the text stream or the timestep embedding gives what the separate operations give: the
+    same tangents, or torch's own error (its derivative of a bf16 layer norm is fp32, which a bf16 projection refuses)."""
+    from torch.autograd import forward_ad
+    block, *args = block_inputs
+
+    def outcome(f):
+        with forward_ad.dual_level():
+            dual = list(args)
+            dual[which] = forward_ad.make_dual(args[which], torch.ones_like(args[which]))
+            try:
+                return [forward_ad.unpack_dual(x).tangent for x in f(*dual)]
+            except RuntimeError as e:
+                return str(e)
+
+    got, want = outcome(block), outcome(lambda *a: _general(block, *a))
+    assert isinstance(got, str) == isinstance(want, str)
+    if isinstance(want, str):
+        assert got == want
+    else:
+        assert any(t is not None for t in want)
+        for a, b in zip(got, want):
+            assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
+
+
+@torch.no_grad()
+def test_a_tangent_of_the_sublayer_output_is_not_dropped(block_inputs):
+    """h + gate * a, with tangents that enter behind the norms."""
+    from torch.autograd import forward_ad
+    from ditango_b200.executor.cogvideox_dit import gated_residual
+    _, h, enc, _, _ = block_inputs
+    a, mod = torch.cat([enc, h], dim=1), torch.randn(2, 6 * 256, device="cuda").to(torch.bfloat16)
+    with forward_ad.dual_level():
+        vo, to = gated_residual(h, enc, forward_ad.make_dual(a, torch.ones_like(a)), mod)
+        gate, e_gate = mod.chunk(6, dim=1)[2::3]
+        assert torch.equal(forward_ad.unpack_dual(vo).tangent, gate[:, None].expand_as(h))
+        assert torch.equal(forward_ad.unpack_dual(to).tangent, e_gate[:, None].expand_as(enc))

@@ -52,3 +52,29 @@ def test_the_fused_path_and_the_general_one_agree_and_hooks_keep_the_general_one
         strided = norm_and_rotate(q.transpose(1, 2).contiguous().transpose(1, 2), k, nq, nk, ang.cos(), ang.sin(), 6)
     for a, b, c in zip(fused, plain, strided):       # the general path rounds to bf16 twice more
         assert (a.float() - b.float()).abs().max() <= 2.0 ** -7 * b.float().abs().max() and torch.equal(b, c)
+
+
+@torch.no_grad()
+def test_tensors_without_an_address_and_tangents_take_the_general_path():
+    from torch.autograd import forward_ad
+    from ditango_b200 import ops
+    from ditango_b200.executor.cogvideox_dit import norm_and_rotate
+    torch.manual_seed(0)
+    q, k = (torch.randn(2, 9, 4, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    nq, nk = (nn.LayerNorm(64, eps=1e-6).cuda().to(torch.bfloat16) for _ in range(2))
+    ang = torch.randn(7, 64, device="cuda")
+    f = lambda a, b: norm_and_rotate(a, b, nq, nk, ang.cos(), ang.sin(), 2)
+    n0 = ops.LaunchLog.count
+    nq.register_forward_hook(lambda m, i, o: None)
+    want = f(q, k)
+    nq._forward_hooks.clear()
+    assert ops.LaunchLog.count == n0
+    for got in (torch.func.vmap(lambda a, b: f(a[None], b[None]))(q, k), torch.func.jvp(f, (q, k), (q, k))[0]):
+        assert all(torch.equal(a.view(b.shape), b) for a, b in zip(got, want))
+    with forward_ad.dual_level():
+        got = f(forward_ad.make_dual(q, torch.ones_like(q)), k)
+        assert forward_ad.unpack_dual(got[0]).tangent is not None and torch.equal(got[1], want[1])
+    for shape in ((0, 9, 4, 64), (2, 9, 0, 64)):
+        e = torch.empty(shape, device="cuda", dtype=torch.bfloat16)
+        assert all(x.shape == shape for x in f(e, e))
+    assert ops.LaunchLog.count == n0
