@@ -107,6 +107,40 @@ def _plain_bf16(device: torch.device, *tensors: torch.Tensor) -> bool:
     return all(x.dtype == torch.bfloat16 and x.device == device and x.is_contiguous() for x in tensors) and _addressable(*tensors)
 
 
+def _rotate_video(x, cos, sin, text_len: int) -> torch.Tensor:
+    return torch.cat([x[:, :text_len], apply_rotary(x[:, text_len:], cos, sin)], dim=1)
+
+
+class _NormRotate(torch.autograd.Function):
+    """The kernel of norm_and_rotate with the gradient of the operations it stands in for: they are run again on the saved
+    inputs."""
+
+    @staticmethod
+    def launch(q, k, q_weight, q_bias, k_weight, k_bias, cos, sin, q_eps, k_eps, text_len):
+        return _engine.norm_rope(q, k, (q_weight, q_bias, q_eps), (k_weight, k_bias, k_eps), cos, sin, text_len)
+
+    @staticmethod
+    def forward(ctx, *args):
+        ctx.save_for_backward(*args[:8])
+        ctx.eps_and_len = args[8:]
+        return _NormRotate.launch(*args)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        q_eps, k_eps, text_len = ctx.eps_and_len
+        with torch.enable_grad(), torch.autocast("cuda", enabled=False):
+            # an alias per argument: a tensor that is passed twice gets each argument's own share
+            args = [x.view_as(x) for x in ctx.saved_tensors]
+            q, k, q_weight, q_bias, k_weight, k_bias, cos, sin = args
+            outs = [_rotate_video(F.layer_norm(x, x.shape[-1:], w, b, eps), cos, sin, text_len)
+                    for x, w, b, eps in ((q, q_weight, q_bias, q_eps), (k, k_weight, k_bias, k_eps))]
+        wanted = [x for x, need in zip(args, ctx.needs_input_grad) if need]
+        pairs = [(o, g) for o, g in zip(outs, grads) if o.requires_grad]
+        got = iter(torch.autograd.grad([o for o, _ in pairs], wanted, [g for _, g in pairs],
+                                       create_graph=torch.is_grad_enabled(), allow_unused=True))
+        return tuple(next(got) if need else None for need in ctx.needs_input_grad)
+
+
 def norm_and_rotate(q, k, norm_q, norm_k, cos, sin, text_len: int) -> Tuple[torch.Tensor, torch.Tensor]:
     """norm_q / norm_k over the heads of q, k [B, S, H, D], then rotary embedding of the tokens behind the first
     text_len.  On a GPU in bf16 this is one kernel over both tensors (fp32 inside, one rounding at the end)."""
@@ -116,12 +150,11 @@ def norm_and_rotate(q, k, norm_q, norm_k, cos, sin, text_len: int) -> Tuple[torc
             all(x.dtype == torch.float32 and x.shape == (q.shape[1] - text_len, D) and x.is_contiguous() and
                 x.device == q.device and (x.numel() == 0 or _addressable(x)) for x in (cos, sin)) and
             not torch.is_autocast_enabled("cuda")):
-        return _engine.norm_rope(q, k, (norm_q.weight, norm_q.bias, norm_q.eps), (norm_k.weight, norm_k.bias, norm_k.eps),
-                                 cos, sin, text_len)
-    q, k = norm_q(q), norm_k(k)
-    q = torch.cat([q[:, :text_len], apply_rotary(q[:, text_len:], cos, sin)], dim=1)
-    k = torch.cat([k[:, :text_len], apply_rotary(k[:, text_len:], cos, sin)], dim=1)
-    return q.contiguous(), k.contiguous()
+        args = (q, k, norm_q.weight, norm_q.bias, norm_k.weight, norm_k.bias, cos, sin, norm_q.eps, norm_k.eps, text_len)
+        if torch.is_grad_enabled() and any(x.requires_grad for x in args[:8]):
+            return _NormRotate.apply(*args)
+        return _NormRotate.launch(*args)
+    return tuple(_rotate_video(x, cos, sin, text_len).contiguous() for x in (norm_q(q), norm_k(k)))
 
 
 def _plain_modulation(h: torch.Tensor, mod: torch.Tensor) -> bool:

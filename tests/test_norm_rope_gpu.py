@@ -78,3 +78,43 @@ def test_tensors_without_an_address_and_tangents_take_the_general_path():
         e = torch.empty(shape, device="cuda", dtype=torch.bfloat16)
         assert all(x.shape == shape for x in f(e, e))
     assert ops.LaunchLog.count == n0
+
+
+@pytest.mark.parametrize("same", [False, True])
+def test_gradients_are_those_of_the_separate_operations(same):
+    """First and second derivatives through the kernel's path and through the general one; also with one tensor as q and k."""
+    from ditango_b200 import ops
+    from ditango_b200.executor.cogvideox_dit import norm_and_rotate
+    torch.manual_seed(0)
+    q, k = (torch.randn(2, 11, 3, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+    k = q if same else k
+    nq, nk = (nn.LayerNorm(64, eps=1e-6).cuda().to(torch.bfloat16) for _ in range(2))
+    nq.weight.data.normal_()
+    ang = torch.randn(7, 64, device="cuda")
+    g = [torch.randn(2, 11, 3, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    inputs = [q, nq.weight, nq.bias, nk.weight, nk.bias] + ([] if same else [k])
+
+    def derivatives():
+        n0 = ops.LaunchLog.count
+        outs = norm_and_rotate(q, k, nq, nk, ang.cos(), ang.sin(), 4)
+        first = torch.autograd.grad(outs, inputs, g[:2], create_graph=True)
+        return ops.LaunchLog.count - n0, list(first) + list(torch.autograd.grad(first[0], inputs[:2], g[2]))
+
+    launches, got = derivatives()
+    nq.register_forward_hook(lambda m, i, o: None)
+    general, want = derivatives()
+    assert (launches, general) == (1, 0)
+    for a, b in zip(got, want):                # the same operations in the same types; sums may be taken in another order
+        assert a.shape == b.shape and (a.float() - b.float()).abs().max() <= 2.0 ** -6 * b.float().abs().max()
+
+
+def test_a_differentiable_attention_behind_the_norms_reaches_the_projections():
+    from ditango_b200.executor.cogvideox_dit import norm_and_rotate
+    torch.manual_seed(0)
+    proj = nn.Linear(64, 64, device="cuda", dtype=torch.bfloat16)
+    nq, nk = (nn.LayerNorm(64, eps=1e-6).cuda().to(torch.bfloat16) for _ in range(2))
+    x = torch.randn(1, 10, 2, 64, device="cuda", dtype=torch.bfloat16)
+    cos, sin = torch.ones(10, 64, device="cuda"), torch.zeros(10, 64, device="cuda")
+    q, k = norm_and_rotate(proj(x), x, nq, nk, cos, sin, 0)
+    nn.functional.scaled_dot_product_attention(*(t.transpose(1, 2) for t in (q, k, x))).float().pow(2).sum().backward()
+    assert all(p.grad is not None and p.grad.abs().sum() > 0 for p in (proj.weight, nq.weight, nk.weight))
