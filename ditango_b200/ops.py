@@ -31,9 +31,15 @@ class LaunchLog:
         cls.events = [] if with_events else None
 
 
+# The raw handle of a device's current stream: building a Stream object around it costs several times the rest of a launch's
+# Python.  The function is not part of torch's public interface; where a build lacks it, the Stream object is used.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr() -> int:
-    # the raw handle: building a Stream object around it costs several times the rest of a launch's Python
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _need_cuda(*ts):

@@ -247,3 +247,14 @@ def test_receive_buffers_are_per_group_and_follow_the_latest_shape():
     A.release_receive_slots(g1)
     assert not any(k[0] == id(g1) for k in A._SLOTS) and any(k[0] == id(g2) for k in A._SLOTS)
     A.release_receive_slots()
+
+
+def test_launch_stream_without_the_raw_handle(monkeypatch):
+    """A torch build that lacks the raw-handle function (it is not public) still gets the current stream."""
+    from ditango_b200 import ops
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(ops, "_raw_stream", None)
+    assert ops._stream_ptr() == 77
+    monkeypatch.setattr(ops, "_raw_stream", lambda device: 100 + device)
+    assert ops._stream_ptr() == 103
