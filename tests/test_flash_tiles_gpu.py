@@ -50,7 +50,7 @@ def test_tile_edges(D, Sq, Sk, scale):
 
 @pytest.mark.parametrize("D", [64, 128])
 def test_rising_scores_rescale_at_every_tile(D):
-    """Scores that rise by more than 2^8 with every key tile."""
+    """Scores whose weights rise 2^4.3-fold with every key tile (a rescale in every second one) and 2^52-fold (in every one)."""
     from ditango_b200 import ops
     q, k, v = _qkv(1, 256, 640, 2, D)
     q = torch.ones_like(q)
