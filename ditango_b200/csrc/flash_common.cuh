@@ -20,8 +20,8 @@ __device__ __forceinline__ void report(int* status, int code) { atomicCAS(status
 
 // Bounded wait that also gives up as soon as any CTA has reported a failure.  The clock is read right after the first
 // failed attempt and not only when it is needed: the pause keeps the waiting warps out of the softmax warps' issue slots
-// (reading it after 64 attempts costs 5 % at D = 64 and 3 % at D = 128; a suspended try_wait or nanosleep in the loop was
-// slower than this too, by up to 4 %).
+// (reading it only after 64 attempts: 119056 tokens at D = 128 150.3 ms against 142.7, a four-chunk ring of 7201 3 % slower,
+// 2 x 17776 tokens at D = 64 1.7 %; a suspended try_wait or nanosleep in the loop was slower than this too, by up to 6 %).
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, int* status, int code) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
@@ -71,7 +71,8 @@ __device__ __forceinline__ uint64_t exp2_mufu2(uint64_t x) {
 }
 
 // ... and on the FMA units, for x <= 127: x = n + f with n = round(x), 2^f on [-1/2, 1/2] by a degree-5 polynomial
-// (least maximum relative error 9.1e-8 with p(0) = 1, weighted least squares iterated to equal ripple), 2^n by
+// (p(0) = 1, weighted least squares iterated to equal ripple; with these coefficients the largest relative error is
+// 1.1e-7, and 1.7e-7 as evaluated here in fp32), 2^n by
 // placing n + 127 in the exponent field.  Below -127 the result is 0; a NaN stays a NaN.
 __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x) {
   float x0, x1;
@@ -128,7 +129,8 @@ __device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, 
 // The rows go through shared memory so that 8 lanes write (and read) the 128 contiguous bytes of a row: a lane that
 // stores its own row touches 32 cache lines per warp instruction, half a sector of each, and the load / store unit then
 // spends a clock per line (32 x 16 instructions x 8 warps for 256 rows of 64 columns, twice that with a state to read).
-// CogVideoX ring on rank 3 of 8 3.91 -> 3.70 ms, its whole sequence 9.65 -> 9.41 ms.  The 16-byte pieces are XOR-swizzled by row, so that neither side has bank conflicts.
+// CogVideoX ring on rank 3 of 8 3.91 -> 3.70 ms, its whole sequence 9.65 -> 9.41 ms.  The 16-byte pieces are XOR-swizzled
+// by row, so that neither side has bank conflicts.
 __device__ __forceinline__ void store_rows32(const FlashParams& p, uint8_t* stage, int64_t tok0, int rows, int64_t col,
                                              const uint32_t (&acc)[32], float w_new, float w_old) {
   const int lane = threadIdx.x & 31;

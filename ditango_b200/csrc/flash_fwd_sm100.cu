@@ -20,13 +20,17 @@
 // at D = 128.  One thread per row and 128 scores per thread: the barrier waits, tensor-memory round trips and
 // hand-overs of a tile are paid once per 128 scores, and the row maximum needs no exchange.  One pair of scores in
 // eight is exponentiated on the FMA units, which takes an eighth of the work off the ex2 unit (16 results per clock and
-// SM: 2048 clocks for the 256 x 128 scores of a step, as much as all MMAs of a step at D = 128); with none the kernel is
-// slower by 2-4 %, with two by 1-3 %, with four by 20 %, the FMA and issue slots then being the bound.
+// SM: 2048 clocks for the 256 x 128 scores of a step, as much as all MMAs of a step at D = 128).  TFLOP/s in short bursts,
+// D = 64 / D = 128: none 857 / 1221, one pair of eight 888 / 1255, two 881 / 1226, four 685 / 1058 (the FMA and issue slots
+// then being the bound).
 //
-// Measured on one B200, launches alone, per step of 128 keys x 256 rows (SM clocks): the MMAs without the softmax 2250
-// at D = 128 and 1430 at D = 64, the softmax without the MMAs 2540 and 2460, both 3050 and 2680.  TFLOP/s against the
-// two kernels with 64-key tiles that this one replaced: D = 64 at 2 x 17776 tokens x 48 heads 922 (before 769), D = 128
-// at 14882 tokens x 24 heads 1286 (1170); sustained, with the board at its power cap, 1186-1220 (1103) at 119056 tokens.
+// Measured on one B200, SM clocks per step of 128 keys x 256 rows (key loop of every CTA, clock register read in front of it
+// and behind it): D = 64 2368, D = 128 2931; in builds with one side left out, the MMAs alone 1280 and 2103, the softmax
+// alone 2357 and 2594.  TFLOP/s, with the two kernels of 64-key tiles that this one replaced in brackets, as a burst of
+// three launches after a pause and back to back for 2.5 s:
+//   D = 64,  2 x 17776 tokens x 48 heads   925 (771) at 1.83 GHz     826 (733) at 1.77 GHz, the board at its power cap
+//   D = 128, 14882 tokens x 24 heads      1283 (1198) at 1.65 GHz   1112 (1034) at 1.59 GHz, power cap
+//   D = 128, 119056 tokens x 24 heads     1225 (1147) on average    1189 (1116) at 1.54 GHz, power cap
 //
 // Running max is kept lazily: O is rescaled only when the max grew by more than 2^8, which bounds every
 // probability by 2^8 and keeps bf16 P exact enough; the final normalisation undoes it.
@@ -47,8 +51,8 @@ constexpr int kRegsOther = 88;      // ... are the 128 x (168 - 88) the third wa
 static_assert(2 * kRegsSoftmax + kRegsOther == 3 * kRegsLaunch, "register split");
 constexpr int kTmaWarp = 8;
 constexpr int kMmaWarp = 9;
-constexpr int kSplit = 64;          // ... of which P's first part covers this many
-constexpr int kPolyPairs = 1;       // of every 8 pairs of scores, exponentiated on the FMA units
+constexpr int kSplit = 64;          // keys of a tile whose probabilities are handed over first
+constexpr int kPolyPairs = 1;       // pairs of every 8 pairs of scores, exponentiated on the FMA units
 
 template <int D>
 struct Cfg {

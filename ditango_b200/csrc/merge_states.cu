@@ -8,9 +8,9 @@
 //
 // A state is kept as loaded (raw bits) until its weight is known.  Its type is only known at run time, so the
 // fp32 and the bf16 load sit in different branches; converting there would make each branch wait for its own load,
-// and the loads of several states would queue behind one another instead of being in flight together (four lanes of 4
-// values with the conversion at the load: fp32 + bf16 at 14882 x 24 x 128 136 us, seven bf16 states and one fp32 at
-// 2 x 6851 x 48 x 128 756 us; as it stands 79 us and 298 us).
+// and the loads of several states would queue behind one another instead of being in flight together (4 values per lane
+// with the conversion at the load: fp32 + bf16 at 14882 x 24 x 128 141 us, seven bf16 states and one fp32 into a bf16 result
+// at 2 x 6851 x 48 x 128 726 us; as it stands 81 us and 306 us; L2 flushed before each launch).
 #include "merge_states.cuh"
 
 #include <math.h>
@@ -212,8 +212,9 @@ static cudaError_t launch_merge_cfg(const MergeParams& p, int G, int sm_count, c
   return cudaGetLastError();
 }
 
-// Rows per thread x states per fetch are chosen so that about eight 16-byte loads are outstanding
-// per thread whatever the number of states: 4 rows x 2 states, 3 x 3, or 2 x 4.
+// Rows per thread x states per fetch are chosen so that eight or nine row pieces are outstanding per thread whatever the
+// number of states: 4 rows x 2 states, 3 x 3, or 2 x 4 (a piece is one 16-byte load in bf16 and two in fp32).  The registers
+// that takes (128) leave four CTAs per SM.
 cudaError_t launch_merge(const MergeParams& p, int head_dim, int sm_count, cudaStream_t stream) {
   const int G = head_dim / 8;
   if (p.rows >= (1ll << 31)) return cudaErrorInvalidValue;

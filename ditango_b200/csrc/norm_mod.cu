@@ -8,8 +8,9 @@
 // per lane and access, all of a row's loads in flight together, the reductions in shuffles), which holds rows of up to
 // 3072 values in registers; wider models keep the separate passes.  The row-independent factors weight * (1 + scale) and
 // bias * (1 + scale) + shift of a sequence are formed once per CTA in shared memory (fp32) and serve all its rows.
-// Measured at 2 x 17776 tokens x 3072: ln_modulate 104 us (437 MB, 4.2 TB/s), gate_add 102 us (655 MB, 6.4 TB/s); the
-// chains they replace took about 400 and 250 us.
+// Measured at 2 x 17776 tokens x 3072, L2 flushed before each launch: ln_modulate 104 us (437 MB, 4.2 TB/s), gate_add 113 us
+// (655 MB, 5.8 TB/s); the chains they replace took about 400 and 250 us.  At 11 and 12 pieces per lane ln_modulate takes 130
+// registers, so that one CTA fits an SM, with 8 of its 64 warps: what holds it below gate_add's rate.
 #include "norm_mod.cuh"
 
 #include "ptx_sm100.cuh"
@@ -19,7 +20,6 @@ namespace dtb {
 namespace {
 
 constexpr int kWarps = 8;
-constexpr int kMaxVec = kModMaxDim / 256;      // 16-byte accesses per lane and row
 
 __device__ __forceinline__ void unpack8(uint4 v, float (&x)[8]) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -155,7 +155,8 @@ static cudaError_t launch_ln(const LnModulateParams& p, dim3 grid, cudaStream_t 
 }
 
 cudaError_t launch_ln_modulate(const LnModulateParams& p, int batch, int sm_count, cudaStream_t stream) {
-  // about four CTAs per SM in all, so that the factors are formed rarely next to the rows they serve
+  // about four CTAs per SM in all per stream, so that the factors are formed rarely next to the rows they serve (how many
+  // of them run at a time is up to the registers: one at 11 and 12 pieces per lane)
   const int longest = p.text_len > p.video_len ? p.text_len : p.video_len;
   const int cap = (4 * sm_count + batch - 1) / batch;
   const int need = (longest + kWarps - 1) / kWarps;
