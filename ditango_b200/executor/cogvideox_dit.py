@@ -254,7 +254,8 @@ class DiTBlock(nn.Module):
 
     def forward(self, h, enc, temb, rope):
         text_len = enc.shape[1]
-        if self.mode != "ulysses" and self.norm1.fuses(h, enc):
+        # (a subclass's or an instance's own _attend takes the streams one by one)
+        if self.mode != "ulysses" and getattr(self._attend, "__func__", None) is DiTBlock._attend and self.norm1.fuses(h, enc):
             x, mod = self.norm1.joint(h, enc, temb)
             h, enc = gated_residual(h, enc, self._attend_joint(x, text_len, rope), mod)
         else:

@@ -180,3 +180,16 @@ def test_a_tangent_of_the_sublayer_output_is_not_dropped(block_inputs):
         gate, e_gate = mod.chunk(6, dim=1)[2::3]
         assert torch.equal(forward_ad.unpack_dual(vo).tangent, gate[:, None].expand_as(h))
         assert torch.equal(forward_ad.unpack_dual(to).tangent, e_gate[:, None].expand_as(enc))
+
+
+@torch.no_grad()
+def test_a_replaced_attention_step_is_called(block_inputs):
+    block, *args = block_inputs
+    seen = []
+
+    def attend(h, enc, rope):
+        seen.append((h.shape, enc.shape))
+        return torch.zeros_like(h), torch.zeros_like(enc)
+    block._attend = attend
+    _close(block(*args), _general(block, *args))
+    assert seen == [(args[0].shape, args[1].shape)] * 2
