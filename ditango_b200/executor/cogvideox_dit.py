@@ -81,18 +81,21 @@ def _unobserved(m: nn.Module, kind: type) -> bool:
                  mod._global_backward_pre_hooks))
 
 
+_PLAIN_TYPES = (torch.Tensor, nn.Parameter)
+
+
 def _addressable(*tensors: torch.Tensor) -> bool:
     """Whether a kernel that is given addresses sees all there is to `tensors`: values in memory of their own (no subclass,
     nothing that torch.func wraps) and no forward-mode tangent, which it would drop.  Alignment: 16 bytes."""
-    for x in tensors:
-        if type(x) not in (torch.Tensor, nn.Parameter):
-            return False
-        try:
+    # (outside of a dual level, the usual case, no tensor has a tangent; the level is not public: without it all are asked)
+    duals = getattr(forward_ad, "_current_level", 0) >= 0
+    try:
+        for x in tensors:
             address = x.data_ptr()
-        except RuntimeError:
-            return False
-        if address == 0 or address % 16 or forward_ad.unpack_dual(x).tangent is not None:
-            return False
+            if type(x) not in _PLAIN_TYPES or address == 0 or address % 16 or (duals and forward_ad.unpack_dual(x).tangent is not None):
+                return False
+    except RuntimeError:        # no storage
+        return False
     return True
 
 
