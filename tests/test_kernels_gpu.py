@@ -227,3 +227,25 @@ def test_drift_accumulate_special_cases():
     acc.zero_()
     ops.drift_accumulate(base.cuda()[1:], (base * 1.1).cuda()[1:], acc)
     assert abs(acc.item() - O.rel_l1(base[1:], (base * 1.1)[1:])) < 1e-6
+
+
+@pytest.mark.parametrize("C,N,B,S", [(16, 1, 1, 1), (16, 1, 1, 1023), (48, 2, 1, 1024), (80, 3, 5, 1025), (768, 8, 2, 341),
+                                     (16 * 1025, 2, 3, 7), (512, 4, 1, 80000)])
+def test_copy_chunks_at_the_edges_of_its_tiles(C, N, B, S):
+    """Vectors that do not fill a tile of 1024, one chunk per vector, chunks larger than a tile, more tiles than one pass of
+    the grid takes."""
+    ops = _ops()
+    x = torch.randint(0, 2 ** 15, (B, S, N, C // 2), device="cuda", dtype=torch.int16).view(torch.bfloat16)
+    out = torch.empty(N, B, S, C // 2, device="cuda", dtype=torch.bfloat16)
+    ops.copy_chunks([(x, out)], C, (N, B, S), (C, S * N * C, N * C), (B * S * C, S * C, C))
+    assert torch.equal(out.view(torch.int16), x.view(torch.int16).permute(2, 0, 1, 3))
+
+
+def test_copy_chunks_counts_beyond_32_bits():
+    """More 16-byte vectors than 32 bits count: an outer dimension of stride 0 copies the same chunks again and again."""
+    ops = _ops()
+    x = torch.randn(3, 5, 4096, device="cuda").to(torch.bfloat16)
+    out = torch.zeros_like(x)
+    C, reps = 4096 * 2, 2 ** 32 // (15 * 512) + 7
+    ops.copy_chunks([(x, out)], C, (reps, 3, 5), (0, 5 * C, C), (0, 5 * C, C))
+    assert torch.equal(out, x)
