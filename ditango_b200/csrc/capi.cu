@@ -265,6 +265,16 @@ DTB_API int dtb_peer_copy_async(void* dst, const void* src, int64_t bytes, void*
   return DTB_OK;
 }
 
+// Which launches take the kernel whose CTAs stay (D = 64): it saves what a CTA spends in front of its key loop and behind it, and
+// is 3 % slower per key tile.  Both sides in us, a CTA per block -> CTAs that stay, for an fp32 result / folded into a state,
+// overlapping the launch before / a bf16 result, 2 sequences x 48 heads:
+//   1111 queries x 1111 keys   75 / 85 / 72 -> 72 / 80 / 66          8888 x 8888   2176 / 2426 / 2356 -> 2162 / 2408 / 2333
+//   2222 x 2222                186 / 209 / 178 -> 178 / 188 / 166    1111 x 17776   739 / 759 / 740 -> 750 / 760 / 746
+//   4444 x 4444                610 / 668 / 602 -> 596 / 623 / 583    8888 x 512, 24 heads   132 / 189 / 125 -> 107 / 137 / 94
+//   600 x 600 (288 blocks)     30.7 / 34.8 / 28.7 -> 31.7 / 34.8 / 29.6
+// A CTA has to get three blocks or so for the saving to show, hence twice the SMs.
+constexpr int kStayMaxKeys = 8192;
+
 static int flash_fwd_impl(const void* q, const void* k, const void* v,
                           int64_t q_tok_stride, int64_t k_tok_stride, int64_t v_tok_stride,
                           void* out, int out_dtype, int64_t out_tok_stride,
@@ -323,8 +333,12 @@ static int flash_fwd_impl(const void* q, const void* k, const void* v,
   p.lse_layout = lse_layout;
   p.accumulate = accumulate ? 1 : 0;
   p.overlap_previous = (launch_flags & DTB_LAUNCH_OVERLAP_PREVIOUS) ? 1 : 0;
-  cudaError_t e = (head_dim == 64) ? dtb::launch_flash<64>(tq, tk, tv, p, static_cast<cudaStream_t>(stream))
-                                   : dtb::launch_flash<128>(tq, tk, tv, p, static_cast<cudaStream_t>(stream));
+  const int64_t blocks = static_cast<int64_t>((seqlen_q + 255) / 256) * num_heads * nseg;
+  const bool stay = head_dim == 64 && blocks > 2 * d->sm_count && seqlen_k <= kStayMaxKeys;
+  const cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const cudaError_t e = stay              ? dtb::launch_flash_persistent(tq, tk, tv, p, s)
+                        : head_dim == 64  ? dtb::launch_flash<64>(tq, tk, tv, p, s)
+                                          : dtb::launch_flash<128>(tq, tk, tv, p, s);
   if (e != cudaSuccess) return fail(DTB_ERR_CUDA, "dtb_flash_fwd launch failed: %s", cudaGetErrorString(e));
   return DTB_OK;
 }

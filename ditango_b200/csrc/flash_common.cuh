@@ -101,15 +101,11 @@ __device__ __forceinline__ int64_t lse_index(const FlashParams& p, int seg, int 
   return (static_cast<int64_t>(seg) * p.num_heads + head) * p.seqlen_q + q_pos;  // [B,H,S]
 }
 
-// Rows of a (segment, head) that has no keys at all: an empty state (out = 0, lse = -inf).  Merging an empty
-// state into an accumulator changes nothing, so with accumulate set nothing is written.  The first 256
-// threads of the CTA cover its 256 query rows.
+// A row of a (segment, head) that has no keys at all: an empty state (out = 0, lse = -inf).  Merging an empty
+// state into an accumulator changes nothing, so with accumulate set nothing is written.
 template <int D>
-__device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, int head, int q_begin, int q_len, int q0) {
-  if (p.accumulate || threadIdx.x >= kQT * kBM) return;
-  const int q_pos = q0 + threadIdx.x;
+__device__ __forceinline__ void write_empty_row(const FlashParams& p, int seg, int head, int q_begin, int q_len, int q_pos) {
   if (q_pos >= q_len) return;
-  grid_dependency_wait();      // the launch before this one may still be writing the same buffers
   const int64_t tok = static_cast<int64_t>(q_begin) + q_pos;
   p.lse[lse_index(p, seg, head, q_pos, tok)] = -INFINITY;
   if (p.out_dtype == 0) {
@@ -120,10 +116,33 @@ __device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, 
     for (int c = 0; c < D / 8; ++c) o[c] = make_uint4(0u, 0u, 0u, 0u);
   }
 }
+// ... for a CTA's 256 query rows, by its first 256 threads.
+template <int D>
+__device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, int head, int q_begin, int q_len, int q0) {
+  if (p.accumulate || threadIdx.x >= kQT * kBM) return;
+  grid_dependency_wait();      // the launch before this one may still be writing the same buffers
+  write_empty_row<D>(p, seg, head, q_begin, q_len, q0 + static_cast<int>(threadIdx.x));
+}
+
+// The state in global memory that 32 consecutive columns of a warp's 32 output rows are merged with: lane i holds 16 bytes
+// of each of the rows i / 8, i / 8 + 4, ... (see store_rows32).
+struct OldRows {
+  float4 v[8];
+};
+__device__ __forceinline__ void load_old_rows32(const FlashParams& p, int64_t tok0, int rows, int64_t col, OldRows& old) {
+  const int lane = threadIdx.x & 31;
+  const int r0 = lane >> 3, piece = lane & 7;
+  const float* src = static_cast<const float*>(p.out) + (tok0 + r0) * p.out_tok_stride + col + piece * 4;
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    old.v[it] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (it * 4 + r0 < rows) old.v[it] = *reinterpret_cast<const float4*>(src + it * 4 * p.out_tok_stride);
+  }
+}
 
 // Final step for 32 consecutive columns of a warp's 32 output rows, executed by the whole warp: lane i holds row i
 // (un-normalised fp32 accumulators `acc`) and its weights.  Scale by w_new, blend with the state already in global memory
-// when accumulating (w_old != 0), store as fp32 or bf16.  `tok0` is the token of the warp's first row, `rows` how many of
+// when accumulating (`old`, used where w_old != 0), store as fp32 or bf16.  `tok0` is the token of the warp's first row, `rows` how many of
 // its rows exist, `col` the element offset of the columns inside a token; `stage` is 4 KB of shared memory of the warp.
 //
 // The rows go through shared memory so that 8 lanes write (and read) the 128 contiguous bytes of a row: a lane that
@@ -132,20 +151,11 @@ __device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, 
 // CogVideoX ring on rank 3 of 8 3.91 -> 3.70 ms, its whole sequence 9.65 -> 9.41 ms.  The 16-byte pieces are XOR-swizzled
 // by row, so that neither side has bank conflicts.
 __device__ __forceinline__ void store_rows32(const FlashParams& p, uint8_t* stage, int64_t tok0, int rows, int64_t col,
-                                             const uint32_t (&acc)[32], float w_new, float w_old) {
+                                             const uint32_t (&acc)[32], const OldRows& old, float w_new, float w_old) {
   const int lane = threadIdx.x & 31;
   const bool f32 = p.out_dtype == 0;
   const int r0 = lane >> 3, piece = lane & 7;
   float* dst = static_cast<float*>(p.out) + (tok0 + r0) * p.out_tok_stride + col + piece * 4;
-  float4 old[8];
-  if (p.accumulate) {
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const float wo = __shfl_sync(0xffffffffu, w_old, it * 4 + r0);
-      old[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (it * 4 + r0 < rows && wo != 0.f) old[it] = *reinterpret_cast<const float4*>(dst + it * 4 * p.out_tok_stride);
-    }
-  }
 #pragma unroll
   for (int i = 0; i < 8; ++i)
     *reinterpret_cast<float4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) =
@@ -161,10 +171,10 @@ __device__ __forceinline__ void store_rows32(const FlashParams& p, uint8_t* stag
       if (p.accumulate) {
         const float wo = __shfl_sync(0xffffffffu, w_old, r);
         if (wo != 0.f) {
-          v.x = fmaf(old[it].x, wo, v.x);
-          v.y = fmaf(old[it].y, wo, v.y);
-          v.z = fmaf(old[it].z, wo, v.z);
-          v.w = fmaf(old[it].w, wo, v.w);
+          v.x = fmaf(old.v[it].x, wo, v.x);
+          v.y = fmaf(old.v[it].y, wo, v.y);
+          v.z = fmaf(old.v[it].z, wo, v.z);
+          v.w = fmaf(old.v[it].w, wo, v.w);
         }
       }
       if (r < rows) *reinterpret_cast<float4*>(dst + it * 4 * p.out_tok_stride) = v;

@@ -456,7 +456,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         uint32_t orow[32];
         tmem_ld32(o_taddr + q * 32, orow);
         tmem_wait_ld<32>(orow);
-        if (rows > 0) store_rows32(p, stage, tok0, rows, static_cast<int64_t>(head) * D + q * 32, orow, w_new, w_old);
+        OldRows old;
+        if (p.accumulate) load_old_rows32(p, tok0, rows, static_cast<int64_t>(head) * D + q * 32, old);
+        if (rows > 0) store_rows32(p, stage, tok0, rows, static_cast<int64_t>(head) * D + q * 32, orow, old, w_new, w_old);
       }
     }
   }

@@ -34,6 +34,11 @@ template <int D>
 cudaError_t launch_flash(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
                          const FlashParams& p, cudaStream_t stream);
 
+// The same for D = 64 by CTAs that stay and take one block of 256 query rows after another (flash_fwd_persistent_sm100.cu).
+// Same tensor maps, same results to the bit.
+cudaError_t launch_flash_persistent(const CUtensorMap& tm_q, const CUtensorMap& tm_k, const CUtensorMap& tm_v,
+                                    const FlashParams& p, cudaStream_t stream);
+
 // Rows of one K / V tile: the tensor maps of k and v must be encoded with boxes of 64 x this many elements
 // (q always uses 64 x 128).
 int flash_kv_box_rows();

@@ -1,0 +1,133 @@
+"""The attention kernel whose CTAs stay and take one block of queries after another, at the sizes where that can go wrong.
+
+A launch at D = 64 with more than two blocks (256 query rows of one head) per SM takes it; the same work head by head stays below
+that and takes the kernel with one CTA per block.  Both do the same arithmetic in the same order, so results agree bit for bit;
+the first cases are also held against softmax in 64 bits.  Tolerances there: probabilities are rounded to bf16 (relative 2^-9)
+before they meet V, so a result differs from exact by at most 2^-9 of the largest |V| plus fp32 accumulation, 2^-8 in all; lse
+is fp32 with exponentials good to 3e-7: |d lse| <= 1e-6 (1 + |lse|)."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _blocks(Sq, H, nseg):
+    return -(-Sq // 256) * H * nseg
+
+
+def _qkv(B, Sq, Sk, H, D, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return tuple(torch.randn(B, S, H, D, generator=g, device="cuda").to(torch.bfloat16) for S in (Sq, Sk, Sk))
+
+
+def _sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def _by_head(q, k, v, **kw):
+    """The same call in launches of one head each."""
+    from ditango_b200 import ops
+    parts = [ops.flash_partial(*(x[..., h:h + 1, :].contiguous() for x in (q, k, v)), **kw) for h in range(q.shape[-2])]
+    return torch.cat([o for o, _ in parts], dim=-2), torch.cat([l for _, l in parts], dim=-2)
+
+
+@pytest.mark.parametrize("D", [64])
+@pytest.mark.parametrize("Sq,Sk", [(257, 1), (300, 63), (512, 64), (257, 65), (300, 127), (256, 128), (600, 129), (300, 200), (256, 256),
+                                   (257, 257), (300, 391), (1000, 640), (300, 1409), (513, 2500)])
+def test_a_full_grid_gives_the_bits_of_its_heads(D, Sq, Sk):
+    from ditango_b200 import ops
+    B, H = 2, 160
+    q, k, v = _qkv(B, Sq, Sk, H, D)
+    assert _blocks(Sq, H, B) > 2 * _sms() >= _blocks(Sq, 1, B)
+    o, l = ops.flash_partial(q, k, v)
+    ho, hl = _by_head(q, k, v)
+    assert torch.equal(o, ho) and torch.equal(l, hl)
+    s = torch.einsum("bqhd,bkhd->bhqk", q[:, :, :3].double(), k[:, :, :3].double()) / math.sqrt(D)
+    want = torch.einsum("bhqk,bkhd->bqhd", torch.softmax(s, -1), v[:, :, :3].double())
+    assert (o[:, :, :3].double() - want).abs().max() <= v.double().abs().max() * 2.0 ** -8
+    want = torch.logsumexp(s, -1)
+    assert ((l[:, :3].double() - want).abs() <= 1e-6 * (1 + want.abs())).all()
+    # folded into a state, overlapping the launch before it; bf16 result; the other lse layout
+    o2, l2 = ops.flash_partial(q, v, k, out=o, lse=l, accumulate=True, overlap_previous=True)
+    for h in (0, H - 1):
+        one = ops.flash_partial(*(x[:, :, h:h + 1].contiguous() for x in (q, k, v)))
+        one = ops.flash_partial(*(x[:, :, h:h + 1].contiguous() for x in (q, v, k)), out=one[0], lse=one[1], accumulate=True)
+        assert torch.equal(o2[:, :, h:h + 1], one[0]) and torch.equal(l2[:, h:h + 1], one[1])
+    b, bl = ops.flash_partial(q, k, v, out_dtype=torch.bfloat16, lse_layout=ops.LSE_BSH)
+    assert torch.equal(b, ho.to(torch.bfloat16)) and torch.equal(bl.transpose(-1, -2), hl)
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [64])
+@pytest.mark.parametrize("keys", ["ragged", "short", "empty"])
+def test_packed_sequences_of_all_lengths(D, keys):
+    """Work items of very different lengths behind one another: no queries, no keys, one key, many tiles; neighbours that are not
+    finite stay outside."""
+    from ditango_b200 import ops
+    H = 24
+    lens_q = [256, 1, 0, 300, 0, 513, 40, 256, 129, 700, 0, 2, 255, 257, 90, 1000]
+    lens_k = dict(ragged=[300, 0, 5, 129, 64, 1, 1300, 0, 15, 16, 17, 640, 128, 255, 0, 513],
+                  short=[1, 2, 15, 16, 17, 31, 32, 33, 47, 63, 64, 65, 100, 127, 3, 1], empty=[0] * 15 + [7])[keys]
+    cu_q, cu_k = (torch.tensor([0] + torch.tensor(n).cumsum(0).tolist(), dtype=torch.int32, device="cuda") for n in (lens_q, lens_k))
+    q, k, v = (x[0] for x in _qkv(1, sum(lens_q), sum(lens_k), H, D, seed=1))
+    assert _blocks(1000, H, len(lens_q)) > 2 * _sms() >= _blocks(1000, 1, len(lens_q))
+    kw = dict(cu_seqlens_q=cu_q, cu_seqlens_k=cu_k, max_seqlen_q=1000, max_seqlen_k=max(lens_k))
+    o, l = ops.flash_partial(q, k, v, **kw)
+    ho, hl = _by_head(q, k, v, **kw)
+    assert torch.equal(o, ho) and torch.equal(l, hl)
+    kb, vb = k.clone(), v.clone()
+    start = int(cu_k[-2])                      # the last sequence's keys are the neighbours of those before
+    kb[start:], vb[start:] = float("nan"), float("inf")
+    ob, lb = ops.flash_partial(q, kb, vb, **kw)
+    n = int(cu_q[-2])
+    assert torch.equal(ob[:n], o[:n]) and torch.equal(lb[:, :n], l[:, :n])
+    # folding further keys into the state: rows without keys keep it
+    ops.flash_partial(q, k, v, out=o, lse=l, accumulate=True, overlap_previous=False, **kw)
+    for s, (a, b) in enumerate(zip(lens_q, lens_k)):
+        if a and not b:
+            rows = slice(int(cu_q[s]), int(cu_q[s + 1]))
+            assert torch.equal(o[rows], ho[rows]) and torch.equal(l[:, rows], hl[:, rows])
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("D", [64])
+def test_rising_scores_and_chains(D):
+    """A reference that has to move at every key tile, over several work items per CTA; a chain of overlapping launches."""
+    from ditango_b200 import ops
+    q, k, v = _qkv(2, 700, 640, 60, D)
+    q = torch.ones_like(q)
+    step = torch.arange(640, device="cuda") // 128
+    for gain in (0.25, 3.0):
+        kk = (k.float() * 0.01 + (gain * 12.0 / math.sqrt(D)) * step[None, :, None, None]).to(torch.bfloat16)
+        o, l = ops.flash_partial(q, kk, v)
+        ho, hl = _by_head(q, kk, v)
+        assert torch.equal(o, ho) and torch.equal(l, hl)
+
+    chunks = [(k[:, i * 100:].contiguous(), v[:, i * 100:].contiguous()) for i in range(5)]
+
+    def chain(overlap):
+        o, l = ops.flash_partial(q, k, v)
+        for kk, vv in chunks:
+            ops.flash_partial(q, kk, vv, out=o, lse=l, accumulate=True, overlap_previous=overlap)
+        return o, l
+    want = chain(False)
+    for _ in range(5):
+        got = chain(True)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert ops.read_status() == 0
+
+
+def test_a_posted_status_ends_the_launch():
+    """CTAs that start after a failure elsewhere do no work, also where they would have taken several items."""
+    from ditango_b200 import _capi, ops
+    q, k, v = _qkv(2, 1000, 500, 60, 64)
+    want = ops.flash_partial(q, k, v)
+    lib = _capi.load()
+    stream = torch.cuda.current_stream().cuda_stream
+    assert lib.dtb_post_status(77, stream) == 0
+    ops.flash_partial(q, k, v)
+    assert lib.dtb_read_status(stream) == 77
+    got = ops.flash_partial(q, k, v)
+    assert ops.read_status() == 0 and torch.equal(got[0], want[0])
