@@ -224,11 +224,15 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
   // The next work item as every role but the producer sees it: its slot, or -1 when there is none.  Slots are given back by
   // one arrival per reading warp.
   uint32_t fetched = 0;
-  auto fetch = [&](const Shared& sh) {
-    const uint32_t slot = fetched % kWork;
-    const bool ok = wait_or_abort(&sh.work_full[slot], (fetched / kWork) & 1, p.status, 51);
-    ++fetched;
-    return ok && sh.s_work[slot].n_tiles >= 0 ? static_cast<int>(slot) : -1;
+  auto take = [&](const Shared& sh, bool there) {
+    const uint32_t slot = fetched++ % kWork;
+    return there && sh.s_work[slot].n_tiles >= 0 ? static_cast<int>(slot) : -1;
+  };
+  auto fetch = [&](const Shared& sh) {                       // by one thread
+    return take(sh, wait_or_abort(&sh.work_full[fetched % kWork], (fetched / kWork) & 1, p.status, 51));
+  };
+  auto fetch_warp = [&](const Shared& sh) {                  // by a whole warp
+    return take(sh, warp_wait_or_abort(&sh.work_full[fetched % kWork], (fetched / kWork) & 1, p.status, 51));
   };
   auto give_back = [&](const Shared& sh, int slot) {         // by a whole warp
     __syncwarp();
@@ -336,7 +340,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       const Shared sh(smem + opaque_zero());
       // (see flash_fwd_sm100.cu: the K step of 16 keys in which a sequence ends holds rows of whatever follows it)
       int it = 0;
-      for (int slot; (slot = fetch(sh)) >= 0;) {
+      for (int slot; (slot = fetch_warp(sh)) >= 0;) {
         const uint32_t use = ((fetched - 1) / kWork) & 1;
         const int n = sh.s_work[slot].n_tiles;
         const int tail = sh.s_work[slot].k_len - (n - 1) * kBN;
@@ -344,9 +348,9 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         if (n > 0 && (tail & 15) != 0) {
           const int stage = (it - 1) % C::kStages;                 // V of the last tile is the last load
           // (the ring slot's barrier is only looked at once this load is the one under way in it)
-          const bool landed = wait_or_abort(&sh.tail_go[slot], use, p.status, 16) &&
-                              wait_or_abort(&sh.kv_full[stage], ((it - 1) / C::kStages) & 1, p.status, 12);
-          if (!__all_sync(0xffffffffu, landed)) break;
+          if (!warp_wait_or_abort(&sh.tail_go[slot], use, p.status, 16) ||
+              !warp_wait_or_abort(&sh.kv_full[stage], ((it - 1) / C::kStages) & 1, p.status, 12))
+            break;
           // whole rows of 128 bytes: the swizzle moves 16-byte pieces inside a row only
           uint8_t* first_row = sh.s_kv + stage * C::kTileBytes + tail * 128;
 #pragma unroll 1
@@ -526,7 +530,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       // The launch before this one (which may still be running if this launch overlaps it) must have completed before its
       // state is read for accumulation or its buffers are written.
       grid_dependency_wait();
-      for (int slot; (slot = fetch(sh)) >= 0;) {
+      for (int slot; (slot = fetch_warp(sh)) >= 0;) {
         const Item w = sh.s_work[slot];
         give_back(sh, slot);
         if (w.n_tiles == 0) {
@@ -550,14 +554,14 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
             if (lane < rows) lse_old = p.lse[li];
             load_old_rows32(p, tok0, rows, col, old);
           }
-          ok = wait_or_abort(&sh.ml_full[tile], item_use, p.status, 42);
+          ok = warp_wait_or_abort(&sh.ml_full[tile], item_use, p.status, 42);
+          if (!ok) break;
           const float2 ml = sh.s_ml[tile * kBM + quarter * 32 + lane];
           __syncwarp();
           if (lane == 0) mbar_arrive(&sh.ml_empty[tile]);
           float w_new, w_old, lse_out;
           merge_weights(p.accumulate != 0, lse_old, (ml.x * c + log2f(ml.y)) * kLn2, ml.y, w_new, w_old, lse_out);
-          ok = ok && wait_or_abort(&sh.o_final[tile], item_use, p.status, 41);
-          ok = __all_sync(0xffffffffu, ok);
+          ok = warp_wait_or_abort(&sh.o_final[tile], item_use, p.status, 41);
           if (!ok) break;
           tc_fence_after();
           if (lane < rows) p.lse[li] = lse_out;
@@ -594,7 +598,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
       uint32_t pv_use = 1;       // parity of PV of the key tile before
       uint32_t items = 0;
       bool ok = true;
-      for (int slot; ok && (slot = fetch(sh)) >= 0;) {
+      for (int slot; ok && (slot = fetch_warp(sh)) >= 0;) {
         const int n_tiles = sh.s_work[slot].n_tiles;
         const int k_len = sh.s_work[slot].k_len;
         give_back(sh, slot);
@@ -603,7 +607,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
         float l = 0.f;           // running sum of exp2((s - m) * c)
         for (int j = 0; j < n_tiles; ++j) {
           const uint32_t s_taddr = lane_base + C::kColS + buf * kBN;   // S(u), then P(u) over its first half
-          ok = wait_or_abort(&sh.s_full[buf], use, p.status, 31 + tile);
+          ok = warp_wait_or_abort(&sh.s_full[buf], use, p.status, 31 + tile);
           if (!ok) break;
           tc_fence_after();
           uint32_t sr[kBN];
@@ -645,7 +649,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
             if (__any_sync(0xffffffffu, grow)) {
               // O is rescaled in place: PV of this Q tile's key tile before must have drained (PV(u) is not issued before this
               // group hands over P(u))
-              ok = wait_or_abort(&sh.pv_done[tile], pv_use, p.status, 33 + tile);
+              ok = warp_wait_or_abort(&sh.pv_done[tile], pv_use, p.status, 33 + tile);
               if (!ok) break;
               tc_fence_after();
               const float f = ex2((m - m_new) * c);
@@ -698,7 +702,8 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __gr
           if (buf >= NB) { buf -= NB; use ^= 1; }
         }
         if (!ok) break;
-        if (items > 0) ok = wait_or_abort(&sh.ml_empty[tile], (items - 1) & 1, p.status, 43);
+        if (items > 0) ok = warp_wait_or_abort(&sh.ml_empty[tile], (items - 1) & 1, p.status, 43);
+        if (!ok) break;          // the rows before these have not been read
         sh.s_ml[tile * kBM + quarter * 32 + lane] = make_float2(m, l);
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.ml_full[tile]);

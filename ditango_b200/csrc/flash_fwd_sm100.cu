@@ -206,8 +206,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if ((tail & 15) != 0 && __all_sync(0xffffffffu, live)) {
         const int it = 2 * n_tiles - 1;                 // V of the last tile is the last load
         const int stage = it % C::kStages;
-        const bool landed = wait_or_abort(&kv_full[stage], (it / C::kStages) & 1, p.status, 12);
-        if (__all_sync(0xffffffffu, landed)) {
+        if (warp_wait_or_abort(&kv_full[stage], (it / C::kStages) & 1, p.status, 12)) {
           // whole rows of 128 bytes: the swizzle moves 16-byte pieces inside a row only
 #pragma unroll 1
           for (int s = 0; s < C::kSlabs; ++s) {
@@ -334,7 +333,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
     for (int j = 0; ok && j < n_tiles; ++j) {
       const uint32_t s_taddr = lane_base + C::kColS + buf * kBN;   // S(u), then P(u) over its first half
-      ok = wait_or_abort(&s_full[buf], use, p.status, 31 + tile);
+      ok = warp_wait_or_abort(&s_full[buf], use, p.status, 31 + tile);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[kBN];
@@ -377,7 +376,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           // O is rescaled in place: PV(u-2), the unit of this Q tile before this one, must have drained (PV(u) is not
           // issued before this group hands over P(u)).  With two buffers S(u) was issued behind PV(u-2), so it has.
           if (NB > 2) {
-            ok = wait_or_abort(&pv_done[tile], (j - 1) & 1, p.status, 33 + tile);
+            ok = warp_wait_or_abort(&pv_done[tile], (j - 1) & 1, p.status, 33 + tile);
             if (!ok) break;
             tc_fence_after();
           }
@@ -430,11 +429,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (buf >= NB) { buf -= NB; use ^= 1; }
     }
 
-    if (ok) ok = wait_or_abort(&o_final[tile], 0, p.status, 41);
+    if (ok) ok = warp_wait_or_abort(&o_final[tile], 0, p.status, 41);
     // Results: the launch before this one (which may still be running if this launch overlaps it) must have
     // completed before its state is read for accumulation or its buffers are written.
     grid_dependency_wait();
-    ok = __all_sync(0xffffffffu, ok);
     if (ok) {
       tc_fence_after();
       const int warp_pos = q0 + tile * kBM + quarter * 32;      // position of the warp's first row
