@@ -40,11 +40,12 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, in
 
 // The same by a whole warp: all of its lanes go on or all of them give up.  (Waiting each for itself, lanes of one warp can see the
 // phase, the status word and the limit at different moments; those that went on would then wait without a limit, at the next
-// operation of the whole warp, for those that had left.)  wait_or_abort is for a single thread.  The vote per key tile costs 0.4 to 0.8 %
-// with a CTA per block at D = 64 (2 x 8888 x 48 heads 2448 -> 2458 us), nothing measurable at D = 128; a vote after
-// wait_or_abort, at the wait or further down, cost 0.8 % there and 0.7 to 1.1 % at D = 128.
+// operation of the whole warp, for those that had left.)  wait_or_abort is for a single thread.
+// The vote costs up to 0.5 % with a CTA per block at D = 64 (74 heads x 512 x 8192: 106.0 -> 106.6 us) and nothing measurable at
+// D = 128.  Asked as "any that failed", as here, the first attempt goes on faster than as "all that passed" (108.7 us there); a vote
+// further down the tile, under the loads of the scores or with that on the rescale, 107.6 and 106.6 us, and 1.2 and 0.1 % at D = 128.
 __device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parity, int* status, int code) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  if (!__any_sync(0xffffffffu, !mbar_try_wait(bar, parity))) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
