@@ -13,6 +13,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -265,15 +266,45 @@ DTB_API int dtb_peer_copy_async(void* dst, const void* src, int64_t bytes, void*
   return DTB_OK;
 }
 
-// Which launches take the kernel whose CTAs stay (D = 64): it saves what a CTA spends in front of its key loop and behind it, and
-// is 3 % slower per key tile.  Both sides in us, a CTA per block -> CTAs that stay, for an fp32 result / folded into a state,
-// overlapping the launch before / a bf16 result, 2 sequences x 48 heads:
-//   1111 queries x 1111 keys   75 / 85 / 72 -> 72 / 80 / 66          8888 x 8888   2176 / 2426 / 2356 -> 2162 / 2408 / 2333
-//   2222 x 2222                186 / 209 / 178 -> 178 / 188 / 166    1111 x 17776   739 / 759 / 740 -> 750 / 760 / 746
-//   4444 x 4444                610 / 668 / 602 -> 596 / 623 / 583    8888 x 512, 24 heads   132 / 189 / 125 -> 107 / 137 / 94
-//   600 x 600 (288 blocks)     30.7 / 34.8 / 28.7 -> 31.7 / 34.8 / 29.6
-// A CTA has to get three blocks or so for the saving to show, hence twice the SMs.
-constexpr int kStayMaxKeys = 8192;
+// Which launches take the kernel whose CTAs stay (D = 64).  It saves what a CTA spends in front of its key loop and behind it, which
+// shows as soon as some SM gets a second block.  us, a CTA per block -> CTAs that stay, for an fp32 result / a bf16 result:
+//    74 heads x 512 x 2222 (148 blocks)    32.9 / 32.4 -> 34.8 / 33.0      48 x 2 x 2222 x 2222     179 / 189 -> 162 / 170
+//   100 heads x 512 x 2222 (200)           61.2 / 60.0 -> 59.0 / 57.5      48 x 2 x 8888 x 8888    2470 / 2430 -> 2396 / 2381
+//   150 heads x 512 x 128  (300)           20.6 / 18.6 -> 17.5 / 15.2      24 x 17776 x 17776      2411 / 2478 -> 2390 / 2460
+//   150 heads x 512 x 2222                 90.8 / 92.3 -> 84.1 / 85.0      24 x 24000 x 24000      4353 / 4342 -> 4341 / 4337
+//   150 heads x 512 x 8192                  312 / 301 -> 293 / 293         24 x 35552 x 35552      9380 / 9336 -> 9362 / 9360
+// and from about 24000 keys on the two are level, hence kStayMaxKeys.
+// A launch that overlaps the one before it needs more blocks: its first CTAs, on the SMs that fall free early, claim blocks while
+// that launch still runs, and up to kWork = 4 of them where an item is short (the ring for K and V holds four key tiles, so that
+// longer ones hold a CTA back), blocks that the SMs which fall free later then miss.  us, folded into a state, overlapping:
+//   512 queries x  128 keys, 300 / 480 / 592 / 700 blocks     22.7 / 35.1 / 40.6 / 54.2 -> 37.0 / 41.2 / 40.3 / 46.3
+//            (without a state, 400 / 480 / 592                17.8 / 22.4 / 27.1 -> 22.7 / 22.4 / 23.2)
+//                  256 keys, 300 / 400 / 480 / 592            25.5 / 32.7 / 38.4 / 47.5 -> 37.5 / 37.4 / 35.6 / 43.1
+//                  384 keys, 300 / 400 / 480                  28.3 / 35.8 / 45.5 -> 35.4 / 36.4 / 38.4
+//                  512 keys, 288 / 300 / 400                  26.5 / 30.8 / 38.6 -> 28.0 / 28.2 / 30.8
+//                 2222 keys, 190 / 250 / 300 / 444            41.2 / 60.1 / 73.1 / 115 -> 43.7 / 57.9 / 66.5 / 104
+//                 8192 keys, 190 / 250 / 350 / 444             145 / 194 / 259 / 333 -> 149 / 190 / 254 / 325
+// Folding a single key tile into a state without overlap is bound by the state's way through the CTA, which eight warps do faster
+// than four: 4 to 9 % slower at 160 to 296 blocks of 64 and 128 keys, between 6 % slower and 5 % faster at 300 to 1776.
+// `blocks` counts what holds queries: the grid of a packed launch has ceil(max_seqlen_q / 256) blocks for each sequence.  The lengths
+// are only known on the device; one sequence is taken to have the maximum, and the last block of each other to be half full.
+// (Blocks without queries cost less to claim than to launch: 16 x 256 queries and keys with max_seqlen_q = 4096, 24 heads,
+// 59.5 -> 40.8 us.)
+constexpr int kStayMaxKeys = 24576;
+
+static bool takes_staying_kernel(int head_dim, bool packed, int nseg, int seqlen_q, int seqlen_k, int64_t total_q, int num_heads,
+                                 bool accumulate, bool overlap, int sm_count) {
+  if (head_dim != 64 || seqlen_k > kStayMaxKeys) return false;
+  int64_t blocks = (static_cast<int64_t>(seqlen_q) + 255) / 256 * nseg * num_heads;
+  if (packed) {
+    const int64_t longest = std::min<int64_t>(seqlen_q, total_q);
+    const int64_t rows = (longest + 255) / 256 * 256 + (total_q - longest) + 128 * static_cast<int64_t>(nseg - 1);
+    blocks = std::min(blocks, rows * num_heads / 256);
+  }
+  const int key_tiles = (seqlen_k + 127) / 128;
+  if (overlap) return blocks > sm_count * static_cast<int64_t>(key_tiles <= 1 && accumulate ? 4 : key_tiles <= 3 ? 3 : 2);
+  return blocks > sm_count && !(accumulate && key_tiles <= 1);
+}
 
 static int flash_fwd_impl(const void* q, const void* k, const void* v,
                           int64_t q_tok_stride, int64_t k_tok_stride, int64_t v_tok_stride,
@@ -333,8 +364,8 @@ static int flash_fwd_impl(const void* q, const void* k, const void* v,
   p.lse_layout = lse_layout;
   p.accumulate = accumulate ? 1 : 0;
   p.overlap_previous = (launch_flags & DTB_LAUNCH_OVERLAP_PREVIOUS) ? 1 : 0;
-  const int64_t blocks = static_cast<int64_t>((seqlen_q + 255) / 256) * num_heads * nseg;
-  const bool stay = head_dim == 64 && blocks > 2 * d->sm_count && seqlen_k <= kStayMaxKeys;
+  const bool stay = takes_staying_kernel(head_dim, cu_seqlens_q != nullptr, nseg, seqlen_q, seqlen_k, total_q, num_heads,
+                                         p.accumulate != 0, p.overlap_previous != 0, d->sm_count);
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   const cudaError_t e = stay              ? dtb::launch_flash_persistent(tq, tk, tv, p, s)
                         : head_dim == 64  ? dtb::launch_flash<64>(tq, tk, tv, p, s)

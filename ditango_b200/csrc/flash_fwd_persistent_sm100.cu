@@ -1,4 +1,4 @@
-// Partial-attention forward at D = 64 for grids larger than the GPU and short key chunks: the tiles, units and arithmetic of
+// Partial-attention forward at D = 64 for grids larger than the GPU (the rule is in capi.cu): the tiles, units and arithmetic of
 // flash_fwd_sm100.cu (256 query rows as two 128-row Q tiles, key tiles of 128, one softmax thread per row), by CTAs that stay
 // and take one block of queries (one (segment, head, 256 rows): a work item) after another.
 //

@@ -1,7 +1,7 @@
 """The attention kernel whose CTAs stay and take one block of queries after another, at the sizes where that can go wrong.
 
-A launch at D = 64 with more than two blocks (256 query rows of one head) per SM takes it; the same work head by head stays below
-that and takes the kernel with one CTA per block.  Both do the same arithmetic in the same order, so results agree bit for bit;
+A launch at D = 64 with enough blocks (256 query rows of one head) takes it; the same work head by head does not have them and
+takes the kernel with one CTA per block.  Both do the same arithmetic in the same order, so results agree bit for bit;
 the first cases are also held against softmax in 64 bits.  Tolerances there: probabilities are rounded to bf16 (relative 2^-9)
 before they meet V, so a result differs from exact by at most 2^-9 of the largest |V| plus fp32 accumulation, 2^-8 in all; lse
 is fp32 with exponentials good to 3e-7: |d lse| <= 1e-6 (1 + |lse|)."""
@@ -38,9 +38,9 @@ def _by_head(q, k, v, **kw):
                                    (257, 257), (300, 391), (1000, 640), (300, 1409), (513, 2500)])
 def test_a_full_grid_gives_the_bits_of_its_heads(D, Sq, Sk):
     from ditango_b200 import ops
-    B, H = 2, 160
+    B, H = 2, 300
     q, k, v = _qkv(B, Sq, Sk, H, D)
-    assert _blocks(Sq, H, B) > 2 * _sms() >= _blocks(Sq, 1, B)
+    assert _blocks(Sq, H, B) > 4 * _sms() and _blocks(Sq, 1, B) <= _sms()
     o, l = ops.flash_partial(q, k, v)
     ho, hl = _by_head(q, k, v)
     assert torch.equal(o, ho) and torch.equal(l, hl)
@@ -72,7 +72,7 @@ def test_packed_sequences_of_all_lengths(D, keys):
                   short=[1, 2, 15, 16, 17, 31, 32, 33, 47, 63, 64, 65, 100, 127, 3, 1], empty=[0] * 15 + [7])[keys]
     cu_q, cu_k = (torch.tensor([0] + torch.tensor(n).cumsum(0).tolist(), dtype=torch.int32, device="cuda") for n in (lens_q, lens_k))
     q, k, v = (x[0] for x in _qkv(1, sum(lens_q), sum(lens_k), H, D, seed=1))
-    assert _blocks(1000, H, len(lens_q)) > 2 * _sms() >= _blocks(1000, 1, len(lens_q))
+    assert sum(-(-n // 256) for n in lens_q) * H > 2 * _sms() and _blocks(1000, 1, len(lens_q)) <= _sms()
     kw = dict(cu_seqlens_q=cu_q, cu_seqlens_k=cu_k, max_seqlen_q=1000, max_seqlen_k=max(lens_k))
     o, l = ops.flash_partial(q, k, v, **kw)
     ho, hl = _by_head(q, k, v, **kw)
@@ -131,3 +131,56 @@ def test_a_posted_status_ends_the_launch():
     assert lib.dtb_read_status(stream) == 77
     got = ops.flash_partial(q, k, v)
     assert ops.read_status() == 0 and torch.equal(got[0], want[0])
+
+
+def _last_kernel(run):
+    """Which of the two kernels the last attention launch of run() was."""
+    from torch.profiler import ProfilerActivity, profile
+    run()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        run()
+        torch.cuda.synchronize()
+    seen = sorted((e for e in prof.events() if "flash_fwd" in e.name), key=lambda e: e.time_range.start)
+    assert seen, "no attention kernel was recorded"
+    return "stays" if "persistent" in seen[-1].name else "leaves"
+
+
+# Blocks per SM (of 512 queries: two blocks a head), keys, folded into a state, overlapping the launch before.
+@pytest.mark.parametrize("per_sm,Sk,accumulate,overlap,want", [
+    (1, 640, False, False, "leaves"), (1.1, 640, False, False, "stays"), (1.1, 640, True, False, "stays"),
+    (1.1, 128, False, False, "stays"), (1.1, 128, True, False, "leaves"), (1.1, 129, True, False, "stays"),
+    (2, 640, True, True, "leaves"), (2.1, 640, True, True, "stays"), (2.1, 385, True, True, "stays"),
+    (3, 384, True, True, "leaves"), (3.1, 384, True, True, "stays"), (3.1, 129, False, True, "stays"),
+    (3, 128, False, True, "leaves"), (3.1, 128, False, True, "stays"), (4, 128, True, True, "leaves"), (4.1, 128, True, True, "stays"),
+    (1.1, 24576, False, False, "stays"), (1.1, 24577, False, False, "leaves")])
+def test_which_kernel_a_launch_takes(per_sm, Sk, accumulate, overlap, want):
+    from ditango_b200 import ops
+    H = int(per_sm * _sms()) // 2
+    q, k, v = _qkv(1, 512, Sk, H, 64)
+    o, l = ops.flash_partial(q, k, v)
+
+    def run():
+        ops.flash_partial(q, k, v, out=o, lse=l)
+        ops.flash_partial(q, k, v, out=o, lse=l, accumulate=accumulate, overlap_previous=overlap)
+    assert _last_kernel(run) == want
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("overlap,H,lens,want", [(True, 24, [1975, 25], "leaves"), (True, 24, [3000, 25], "stays"),
+                                                 (False, 24, [1000, 25], "leaves"), (False, 48, [500, 25], "leaves"),
+                                                 (False, 24, [1600, 25], "stays"), (True, 48, [1300, 25], "stays")])
+def test_blocks_without_queries_do_not_count(overlap, H, lens, want):
+    """A valid and a pad sequence: almost half of the grid has no queries."""
+    from ditango_b200 import ops
+    cu = torch.tensor([0, lens[0], sum(lens)], dtype=torch.int32, device="cuda")
+    q, k, v = (x[0] for x in _qkv(1, sum(lens), sum(lens), H, 64))
+    kw = dict(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=lens[0], max_seqlen_k=lens[0])
+    assert _blocks(lens[0], H, 2) > (2 if overlap else 1) * _sms()
+    o, l = ops.flash_partial(q, k, v, **kw)
+
+    def run():
+        ops.flash_partial(q, k, v, out=o, lse=l, **kw)
+        ops.flash_partial(q, k, v, out=o, lse=l, accumulate=True, overlap_previous=overlap, **kw)
+    assert _last_kernel(run) == want
+    assert ops.read_status() == 0
