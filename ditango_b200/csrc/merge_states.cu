@@ -227,15 +227,16 @@ cudaError_t launch_merge(const MergeParams& p, int head_dim, int sm_count, cudaS
 
 // ------------------------------------------------------------------------------------------------
 // Strided chunk copy (head <-> sequence re-layouts around the Ulysses all-to-all).
-// The 16-byte vectors of all chunks are numbered through; a thread copies kCopyUnroll of them, a block apart, whose loads are
-// all in flight before the first store.  Bound by HBM once the index arithmetic is out of the way: Index is 32 bits where the
-// vectors can be counted in it, since three 64-bit divisions per vector, with one load in flight per thread, took longer than
-// the copy.  The stores are ordinary ones: what reads the result (the exchange, the attention kernel) comes next and finds
-// part of it in L2.  CogVideoX Ulysses call of one rank of 8 (four re-layouts of 27 to 82 MB): 1345 -> 1315 us.
+// The 16-byte vectors of all chunks are numbered through; a thread copies Unroll of them, a block apart, whose loads are all in
+// flight before the first store (one for small copies: see launch_copy_chunks).  Bound by HBM once the index arithmetic is out of the way: Index is 32 bits where the vectors can
+// be counted in it, since three 64-bit divisions per vector, with one load in flight per thread, took longer than the copy.  The
+// stores are ordinary ones: what reads the result (the exchange, the attention kernel) comes next and finds part of it in L2.
+// us (bytes moved per time), L2 flushed before each launch: the re-layouts of a CogVideoX Ulysses call of one rank of 8, 164 MB
+// 38.9 (4.2 TB/s) -> 32.8 (5.0) and 55 MB 18.5 (3.0) -> 16.4 (3.3); 437 MB 88.1 (5.0) -> 73.7 (5.9).
 constexpr int kCopyThreads = 256;
 constexpr int kCopyUnroll = 4;
 
-template <typename Index>
+template <typename Index, int Unroll>
 __global__ void __launch_bounds__(kCopyThreads) copy_chunks_kernel(const CopyParams p) {
   const int pair = blockIdx.y;
   const uint8_t* src = static_cast<const uint8_t*>(p.src[pair]);
@@ -243,12 +244,12 @@ __global__ void __launch_bounds__(kCopyThreads) copy_chunks_kernel(const CopyPar
   const Index vec_per_chunk = static_cast<Index>(p.chunk_bytes >> 4);
   const Index n1 = static_cast<Index>(p.n1), n2 = static_cast<Index>(p.n2);
   const Index total = static_cast<Index>(p.n0) * n1 * n2 * vec_per_chunk;
-  constexpr Index kTile = kCopyThreads * kCopyUnroll;
+  constexpr Index kTile = kCopyThreads * Unroll;
   for (Index tile = static_cast<Index>(blockIdx.x); tile < (total + (kTile - 1)) / kTile; tile += gridDim.x) {
-    uint4 val[kCopyUnroll];
-    uint8_t* to[kCopyUnroll];
+    uint4 val[Unroll];
+    uint8_t* to[Unroll];
 #pragma unroll
-    for (int u = 0; u < kCopyUnroll; ++u) {
+    for (int u = 0; u < Unroll; ++u) {
       const Index i = tile * kTile + static_cast<Index>(u * kCopyThreads + threadIdx.x);
       to[u] = nullptr;
       if (i < total) {
@@ -263,23 +264,31 @@ __global__ void __launch_bounds__(kCopyThreads) copy_chunks_kernel(const CopyPar
       }
     }
 #pragma unroll
-    for (int u = 0; u < kCopyUnroll; ++u)
+    for (int u = 0; u < Unroll; ++u)
       if (to[u] != nullptr) *reinterpret_cast<uint4*>(to[u]) = val[u];
   }
+}
+
+template <typename Index, int Unroll>
+static cudaError_t launch_copy_chunks_cfg(const CopyParams& p, int npairs, int64_t tiles, cudaStream_t stream) {
+  copy_chunks_kernel<Index, Unroll><<<dim3(static_cast<unsigned>(tiles), npairs), kCopyThreads, 0, stream>>>(p);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_copy_chunks(const CopyParams& p, int npairs, int sm_count, cudaStream_t stream) {
   constexpr int64_t kTile = kCopyThreads * kCopyUnroll;
   const int64_t total = p.n0 * p.n1 * p.n2 * (p.chunk_bytes >> 4);
+  // Up to four tiles for every SM, one vector per thread: more warps in flight count for more there.  us per launch, back to back,
+  // four vectors -> one: 0.2 MB moved 2.6 -> 1.7, 3.2 MB 2.6 -> 2.0, 5.2 MB 3.2 -> 2.4, 12.6 MB 3.8 -> 3.6, 22.9 MB 4.9 -> 5.3,
+  // 54.6 MB 9.0 -> 10.8.
+  if (total <= 4 * sm_count * kTile)
+    return launch_copy_chunks_cfg<uint32_t, 1>(p, npairs, (total + kCopyThreads - 1) / kCopyThreads, stream);
   const int64_t tiles = (total + kTile - 1) / kTile;
   const int64_t cap = static_cast<int64_t>(sm_count) * 64;
-  const int bx = static_cast<int>(tiles < 1 ? 1 : tiles < cap ? tiles : cap);
+  const int64_t grid = tiles < cap ? tiles : cap;
   // (a thread's index goes one grid past the last vector before it stops)
-  if (total + cap * kTile < (1ll << 31))
-    copy_chunks_kernel<uint32_t><<<dim3(bx, npairs), kCopyThreads, 0, stream>>>(p);
-  else
-    copy_chunks_kernel<uint64_t><<<dim3(bx, npairs), kCopyThreads, 0, stream>>>(p);
-  return cudaGetLastError();
+  if (total + cap * kTile < (1ll << 31)) return launch_copy_chunks_cfg<uint32_t, kCopyUnroll>(p, npairs, grid, stream);
+  return launch_copy_chunks_cfg<uint64_t, kCopyUnroll>(p, npairs, grid, stream);
 }
 
 }  // namespace dtb

@@ -230,10 +230,10 @@ def test_drift_accumulate_special_cases():
 
 
 @pytest.mark.parametrize("C,N,B,S", [(16, 1, 1, 1), (16, 1, 1, 1023), (48, 2, 1, 1024), (80, 3, 5, 1025), (768, 8, 2, 341),
-                                     (16 * 1025, 2, 3, 7), (512, 4, 1, 80000)])
+                                     (16 * 1025, 2, 3, 7), (512, 4, 1, 80000), (768, 8, 2, 789), (768, 8, 2, 790)])
 def test_copy_chunks_at_the_edges_of_its_tiles(C, N, B, S):
-    """Vectors that do not fill a tile of 1024, one chunk per vector, chunks larger than a tile, more tiles than one pass of
-    the grid takes."""
+    """Vectors that do not fill a tile, one chunk per vector, chunks larger than a tile, more tiles than one pass of the grid takes,
+    both sides of the line (on 148 SMs) up to which a thread copies one vector."""
     ops = _ops()
     x = torch.randint(0, 2 ** 15, (B, S, N, C // 2), device="cuda", dtype=torch.int16).view(torch.bfloat16)
     out = torch.empty(N, B, S, C // 2, device="cuda", dtype=torch.bfloat16)
