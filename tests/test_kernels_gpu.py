@@ -241,11 +241,15 @@ def test_copy_chunks_at_the_edges_of_its_tiles(C, N, B, S):
     assert torch.equal(out.view(torch.int16), x.view(torch.int16).permute(2, 0, 1, 3))
 
 
-def test_copy_chunks_counts_beyond_32_bits():
-    """More 16-byte vectors than 32 bits count: an outer dimension of stride 0 copies the same chunks again and again."""
+@pytest.mark.parametrize("order", ["outer", "inner"])
+def test_copy_chunks_counts_beyond_32_bits(order):
+    """More 16-byte vectors than 32 bits count: a dimension of stride 0 copies the same chunks again and again.  The count cut to 32
+    bits is less than one pass over the chunks, and leaves the rest of the result as it was."""
     ops = _ops()
     x = torch.randn(3, 5, 4096, device="cuda").to(torch.bfloat16)
     out = torch.zeros_like(x)
-    C, reps = 4096 * 2, 2 ** 32 // (15 * 512) + 7
-    ops.copy_chunks([(x, out)], C, (reps, 3, 5), (0, 5 * C, C), (0, 5 * C, C))
+    C, reps = 4096 * 2, 2 ** 32 // (15 * 512) + 1
+    assert 0 < reps * 15 * 512 - 2 ** 32 < 15 * 512
+    n, stride = ((reps, 3, 5), (0, 5 * C, C)) if order == "outer" else ((3, 5, reps), (5 * C, C, 0))
+    ops.copy_chunks([(x, out)], C, n, stride, stride)
     assert torch.equal(out, x)
