@@ -50,7 +50,8 @@ def test_a_full_grid_gives_the_bits_of_its_heads(D, Sq, Sk):
     want = torch.logsumexp(s, -1)
     assert ((l[:, :3].double() - want).abs() <= 1e-6 * (1 + want.abs())).all()
     # folded into a state, overlapping the launch before it; bf16 result; the other lse layout
-    o2, l2 = ops.flash_partial(q, v, k, out=o, lse=l, accumulate=True, overlap_previous=True)
+    o2, l2 = ops.flash_partial(q, k, v)
+    ops.flash_partial(q, v, k, out=o2, lse=l2, accumulate=True, overlap_previous=True)
     for h in (0, H - 1):
         one = ops.flash_partial(*(x[:, :, h:h + 1].contiguous() for x in (q, k, v)))
         one = ops.flash_partial(*(x[:, :, h:h + 1].contiguous() for x in (q, v, k)), out=one[0], lse=one[1], accumulate=True)
@@ -127,8 +128,10 @@ def test_a_posted_status_ends_the_launch():
     lib = _capi.load()
     stream = torch.cuda.current_stream().cuda_stream
     assert lib.dtb_post_status(77, stream) == 0
-    ops.flash_partial(q, k, v)
+    o, l = torch.full_like(want[0], 5.0), torch.full_like(want[1], 5.0)
+    ops.flash_partial(q, k, v, out=o, lse=l)
     assert lib.dtb_read_status(stream) == 77
+    assert (o == 5.0).all() and (l == 5.0).all()
     got = ops.flash_partial(q, k, v)
     assert ops.read_status() == 0 and torch.equal(got[0], want[0])
 
@@ -183,4 +186,62 @@ def test_blocks_without_queries_do_not_count(overlap, H, lens, want):
         ops.flash_partial(q, k, v, out=o, lse=l, **kw)
         ops.flash_partial(q, k, v, out=o, lse=l, accumulate=True, overlap_previous=overlap, **kw)
     assert _last_kernel(run) == want
+    assert ops.read_status() == 0
+
+
+def test_a_chain_through_both_kernels():
+    """Overlapping launches of which some take one kernel and some the other: each waits for the one before it and, through it, for
+    all others."""
+    from ditango_b200 import ops
+    H = int(2.1 * _sms()) // 2
+    chunks = [_qkv(1, 512, Sk, H, 64, seed=i) for i, Sk in enumerate([640, 300, 1000, 128, 129, 640, 513, 1])]
+    q = chunks[0][0]
+
+    def chain(overlap):
+        o, l = ops.flash_partial(q, *chunks[0][1:])
+        for _, k, v in chunks[1:]:
+            ops.flash_partial(q, k, v, out=o, lse=l, accumulate=True, overlap_previous=overlap)
+        return o, l
+    want = chain(False)
+    torch.cuda.synchronize()
+    for _ in range(10):
+        got = chain(True)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert ops.read_status() == 0
+
+
+def test_views_of_a_fused_projection():
+    """q, k and v one behind the other in each token, the result among other things in a row of its own."""
+    from ditango_b200 import ops
+    B, S, H = 2, 700, 60
+    x = torch.randn(B, S, 3, H, 64, device="cuda").to(torch.bfloat16)
+    q, k, v = x.unbind(2)
+    want = ops.flash_partial(*(t.contiguous() for t in (q, k, v)))
+    for dtype in (torch.float32, torch.bfloat16):
+        rows = torch.full((B, S, 2 * H, 64), 7.0, device="cuda", dtype=dtype)
+        o, l = ops.flash_partial(q, k, v, out=rows[:, :, H:])
+        assert torch.equal(o, want[0].to(dtype)) and torch.equal(l, want[1]) and (rows[:, :, :H] == 7.0).all()
+    rows = torch.full((B, S, 2 * H, 64), 7.0, device="cuda")
+    rows[:, :, :H] = want[0]
+    l = want[1].clone()
+    ops.flash_partial(q, v, k, out=rows[:, :, :H], lse=l, accumulate=True)
+    ops.flash_partial(*(t.contiguous() for t in (q, v, k)), out=want[0], lse=want[1], accumulate=True)
+    assert torch.equal(rows[:, :, :H], want[0]) and torch.equal(l, want[1]) and (rows[:, :, H:] == 7.0).all()
+    assert ops.read_status() == 0
+
+
+def test_two_streams_at_once():
+    from ditango_b200 import ops
+    work = [_qkv(2, 600, 500 + 300 * i, 60, 64, seed=i) for i in range(2)]
+    want = [ops.flash_partial(*w) for w in work]
+    streams = [torch.cuda.Stream() for _ in work]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(10):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(ops.flash_partial(*work[i]))
+    torch.cuda.synchronize()
+    for w, results in zip(want, got):
+        assert all(torch.equal(o, w[0]) and torch.equal(l, w[1]) for o, l in results)
     assert ops.read_status() == 0

@@ -126,10 +126,21 @@ def test_units_run_through_all_items(replay, items):
             for tile in range(2):
                 want += [0 if j == 0 and kk == 0 else 1 for kk in range(n)]
     assert acc == want
+    # where in tensor memory: S(u) in buffer u mod 3, P(u) from there, 8 columns a K step, into the O of its Q tile
+    assert [int(e[1]) for e in ev if e[0] == "S"] == [u % 3 * 128 for u in range(units) for _ in range(4)]
+    at = []
+    u = 0
+    for s in steps:
+        for n in s:
+            for tile in range(2):
+                at += [(384 + 64 * tile, u % 3 * 128 + 8 * kk) for kk in range(n)]
+                u += 1
+    assert [(int(e[1]), int(e[2])) for e in pv] == at
     # S of a unit is behind PV of the unit three before
     s_seen = pv_seen = 0
     for e in ev:
         if e[:2] == ["commit", "s_full"]:
+            assert int(e[2]) == s_seen % 3
             assert s_seen < 3 or pv_seen > s_seen - 3
             s_seen += 1
         if e[:2] == ["wait", "p_hi"]:
