@@ -1,5 +1,6 @@
-// Pieces of the partial-attention forward kernel (flash_fwd_sm100.cu) that are not its schedule: tile geometry, the
-// bounded barrier wait, the status word, packed fp32 arithmetic, the two exponentials, the lse layouts, the epilogue.
+// Pieces of the partial-attention forward kernels (flash_fwd_sm100.cu, flash_fwd_persistent_sm100.cu) that are not their schedule:
+// tile geometry, the bounded barrier waits, the status word, packed fp32 arithmetic, the two exponentials, the lse layouts, the
+// epilogue.
 #pragma once
 #include "flash_fwd_sm100.cuh"
 #include "ptx_sm100.cuh"
@@ -121,8 +122,8 @@ __device__ __forceinline__ int64_t lse_index(const FlashParams& p, int seg, int 
   return (static_cast<int64_t>(seg) * p.num_heads + head) * p.seqlen_q + q_pos;  // [B,H,S]
 }
 
-// A row of a (segment, head) that has no keys at all: an empty state (out = 0, lse = -inf).  Merging an empty
-// state into an accumulator changes nothing, so with accumulate set nothing is written.
+// A row of a (segment, head) that has no keys at all: an empty state (out = 0, lse = -inf).  Not for a launch that folds into a
+// state (callers see to that): merging an empty state changes nothing.
 template <int D>
 __device__ __forceinline__ void write_empty_row(const FlashParams& p, int seg, int head, int q_begin, int q_len, int q_pos) {
   if (q_pos >= q_len) return;
@@ -146,8 +147,9 @@ __device__ __forceinline__ void write_empty_rows(const FlashParams& p, int seg, 
 
 // The state in global memory that 32 consecutive columns of a warp's 32 output rows are merged with: lane i holds 16 bytes
 // of each of the rows i / 8, i / 8 + 4, ... (see store_rows32).  Read whatever its weight turns out to be, so that the loads do
-// not queue behind that of the lse; a state of weight 0 is not used.  (Behind the weight, a launch folded into a state:
-// 2 x 2222 rows x 48 x 64 206 -> 194 us, 7201 x 24 x 128 625 -> 613.)
+// not queue behind that of the lse; a state of weight 0 is not used.  (Reads behind the weight -> as here, a launch with
+// a CTA per block folded into a state, overlapping the one before: 1024 x 24 x 128 20.9 -> 20.5 us, 2 x 1111 x 24 x 128 44.7 -> 44.0,
+// 2 x 2222 x 48 x 64 192.7 -> 191.9.)
 struct OldRows {
   float4 v[8];
 };
@@ -164,8 +166,8 @@ __device__ __forceinline__ void load_old_rows32(const FlashParams& p, int64_t to
 
 // Final step for 32 consecutive columns of a warp's 32 output rows, executed by the whole warp: lane i holds row i
 // (un-normalised fp32 accumulators `acc`) and its weights.  Scale by w_new, blend with the state already in global memory
-// when accumulating (`old`, used where w_old != 0), store as fp32 or bf16.  `tok0` is the token of the warp's first row, `rows` how many of
-// its rows exist, `col` the element offset of the columns inside a token; `stage` is 4 KB of shared memory of the warp.
+// when accumulating (`old`, used where w_old != 0), store as fp32 or bf16.  `tok0` is the token of the warp's first row, `rows` how
+// many of its rows exist, `col` the element offset of the columns inside a token; `stage` is 4 KB of shared memory of the warp.
 //
 // The rows go through shared memory so that 8 lanes write (and read) the 128 contiguous bytes of a row: a lane that
 // stores its own row touches 32 cache lines per warp instruction, half a sector of each, and the load / store unit then

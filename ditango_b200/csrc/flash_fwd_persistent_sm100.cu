@@ -14,18 +14,25 @@
 // launch, tensor-memory allocation, first loads, then the read of the state it is merged with and the stores, all with idle
 // tensor and softmax units.  Here the next item's queries and first keys are loaded and its first scores computed while the
 // softmax warps finish the item before it, and results leave by warps of their own.
-// What is left of the register file for the softmax warps (176 each) and the issuer's longer way through its loop cost 3 % per
-// key tile, so that one CTA per block stays ahead where the loop is long, and at D = 128 (O takes half of tensor memory and
-// the board is at its power cap, where idle phases let the clock recover: 1203 to 1255 TFLOP/s against 1273 to 1287 at
-// 14882 rows x 24 heads).  Measured: see the rule in capi.cu.
+// Per key tile the two are level (512 queries x 296 heads, four blocks per SM, 4096 -> 16384 keys: +640 us with a CTA per block, +639
+// here), though the softmax warps have 176 registers here and 208 there; what is saved is 3 to 5 us a block.  At D = 128 O takes
+// half of tensor memory and the board is at its power cap, where idle phases let the clock recover: a version of this kernel for it
+// reached 1203 to 1255 TFLOP/s at 14882 rows x 24 heads against 1273 to 1287.  Which launches come here: see the rule in capi.cu.
 //
 // Work items.  The grid has one block per item, as if every block were to run.  A CTA claims further blocks by cluster launch
 // control, which hands out blocks that have not started: items go to whichever CTA is free (a static share would wait for SMs
 // that other streams' kernels hold), nothing is counted in memory, and a launch that overlaps this one starts when the last
 // block has started or been claimed.
 //
-// Every barrier has a role that waits for each of its phases before the next one can complete; what a slow role could fall
-// behind on (v_tail, tail_go) has a barrier per work slot, and slots are reused only when every role has given them back.
+// Every phase of a barrier is over for all that look at it before the next one can complete.  Most have a role that waits for each
+// phase.  pv_done is only waited for when a reference moves, but PV(u) needs P(u), which the warps that look at it hand over behind
+// that: it is never a phase ahead of them.  What a slow role could fall behind on (v_tail, tail_go) has a barrier per work slot, and
+// slots are reused only when every role has given them back.
+//
+// Launches that overlap.  The result warps wait for the launch before this one to complete before they touch the state, and the
+// bounded waits of the other roles (work_empty, o_free, ml_empty) go on meanwhile: what is left of that launch when the first CTA of
+// this one starts, at most the blocks that its CTAs have under way, has to take less than their second.  A block takes 13 us per 1000
+// keys.
 #include "flash_common.cuh"
 
 #include <mutex>
