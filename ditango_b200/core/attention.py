@@ -81,11 +81,12 @@ class proAttention:
     # the attention launch before it is finishing (ops.flash_partial); that is allowed when only event waits /
     # records were queued on the stream since that launch.
     #   "auto"  overlap launches of less than OVERLAP_MAX_FLOPS (short ones, where gap and tail are a visible share:
-    #           seven launches of 2 x 2222 rows x 48 heads at D = 64 1.46 -> 1.35 ms, three of 2 x 4444 rows 1.95 -> 1.90),
+    #           seven launches of 2 x 2222 rows x 48 heads at D = 64 1.36 -> 1.30 ms, three of 2 x 4444 rows 2.01 -> 1.98),
     #           and only on transports whose wait for an incoming chunk is an event wait (the group says so:
     #           `wait_is_event_only`).  The line was drawn with an earlier attention kernel, which lost about 1 % above
     #           it (at D = 128 the board is at its power cap, where an idle tail lets the clock recover).  With the
-    #           present one, at 24 heads of D = 128, overlapping gives 2-3 % at 14882 rows, 1 % at 29764 and 0-1 % at 7441;
+    #           present ones, at 24 heads of D = 128, overlapping gives 3-4 % at 14882 rows, 2-3 % at 7201 and 7441 and
+    #           nothing at 29764;
     #   True    overlap every launch that may.  On a transport that copies on the compute stream when it waits,
     #           the own chunk is attended first, then ALL incoming chunks are waited for, then the remaining
     #           launches go back to back;

@@ -24,6 +24,9 @@
 // D = 64 / D = 128: none 857 / 1221, one pair of eight 888 / 1255, two 881 / 1226, four 685 / 1058 (the FMA and issue slots
 // then being the bound).
 //
+// Launches at D = 64 with enough blocks go to flash_fwd_persistent_sm100.cu (the rule is in capi.cu), those of the following
+// figures among them; they were taken before the waits of whole warps voted (up to 0.5 % at D = 64, nothing at D = 128).
+//
 // Measured on one B200, SM clocks per step of 128 keys x 256 rows (key loop of every CTA, clock register read in front of it
 // and behind it): D = 64 2368, D = 128 2931; in builds with one side left out, the MMAs alone 1280 and 2103, the softmax
 // alone 2357 and 2594.  TFLOP/s, with the two kernels of 64-key tiles that this one replaced in brackets, as a burst of
